@@ -456,6 +456,7 @@ __device__ __forceinline__ u32 near_id(const NearSet& N, const SlabSet& D, cplx 
     for (int probe = 0; probe < kNearSlots; ++probe) {
         const u64 seen = N.keys[h];
         if (seen == key) {
+            __threadfence_block();   // the id and the value were written before the key
             const u32 id = N.ids[h];
             const double2 w = N.dict[id];
             if (__double_as_longlong(w.x) == __double_as_longlong(v.re) &&
