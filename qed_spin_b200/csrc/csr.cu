@@ -1046,7 +1046,6 @@ void build_slices(qb_csr* A, uint64_t max_bytes) {
     k_slice<<<static_cast<unsigned>((A->rows + 255) / 256), 256>>>(A->rows, A->row_ptr.p, A->col_idx.p, A->ids.p, cb,
                                                                    A->slices.p);
     cuda_check(cudaGetLastError(), "CSR slices");
-    cuda_check(cudaStreamSynchronize(nullptr), "CSR slices");
 }
 
 // ... and at most this much scratch, an eighth of the free memory at most.
@@ -1201,6 +1200,9 @@ int csr_build(const qb_sector* row, const qb_sector* col, const qb_program* prog
         if (narrow ? build_slabs<u32>(row, col, prog, max_bytes, A.get())
                    : build_slabs<u64>(row, col, prog, max_bytes, A.get())) {
             if (slices) build_slices(A.get(), max_bytes);
+            // the last copies (device to device: the host does not wait for them) and the slices are queued on this
+            // thread's stream, and the matrix may be read on any other as soon as the call returns
+            cuda_check(cudaStreamSynchronize(nullptr), "CSR build");
             *out = A.release();
             return;
         }

@@ -1,7 +1,7 @@
 """The one-walk CSR build of large sectors (from 65,536 rows) against the oracle's merged rows, bit for bit: real and complex
 characters, rows with repeated columns (a dihedral group with spin flip), an operator between two sectors, no symmetry,
-64-bit states; and what it hands to the general path: more than 256 values, a budget that holds the merged entries
-only."""
+64-bit states; what it hands to the general path: more than 256 values, a budget that holds the merged entries
+only; and that the matrix is complete when the call returns, for a stream that waits for no other."""
 import numpy as np
 import pytest
 
@@ -79,3 +79,52 @@ def test_budget_of_the_merged_entries():
         assert np.array_equal(a.view(np.uint32), b.view(np.uint32))
     with pytest.raises(ResourceLimit):
         D.Csr(S, S, P, max_bytes=need - 1)
+
+
+def _projected(n):
+    """Flips of a bond that act only with the next site up: half the entries a row emits are exact zeros, dropped."""
+    prods = ops.xxz_products(lat.chain_bonds(n), 0.0, 0.7)
+    for i in range(n):
+        for a, b in ((i, (i + 1) % n), ((i + 1) % n, i)):
+            prods += [("+-", [a, b], 0.25), ("+-z", [a, b, (i + 2) % n], 0.5)]
+    return ops.row_program(ops.from_products(n, prods))
+
+
+@pytest.mark.parametrize("name", ["projected", "no room for slices"])
+def test_matrix_is_complete_on_return(name):
+    """Applied at once on a non-blocking stream, bit for bit against the same entries uploaded. "projected" ends with the
+    trim of a third of its entries' room, gigabytes-long copies on a large sector; without slices no kernel follows it."""
+    from qed_spin_b200 import device as D
+    n = 24
+    S = D.Sector(lat.chain_sector(n, 12, 3))
+    P = D.Program(_projected(n) if name == "projected" else ops.row_program(_chain(n)))
+    A = D.Csr(S, S, P)
+    info = A.info()
+    U = D.Csr.upload(S, S, *A.download())
+    # the slab build wants room for the entries before the merge; one byte less than the sliced copy's room leaves it out
+    reps = S.reps()[0]
+    flips = sum(int((((reps >> np.uint64(i)) ^ (reps >> np.uint64((i + 1) % n))) & np.uint64(1)).sum()) for i in range(n))
+    unmerged = (S.dim + 1) * 8 + ((flips + S.dim + 3) & ~3) * 5 + 256 * 16
+    budget = max(unmerged, (S.dim + 1) * 8 + info["nnz"] * 9 - 1)
+    sliced = info["bytes"] > (S.dim + 1) * 8 + info["nnz"] * 8
+    assert sliced
+    if name == "projected":
+        assert flips > 1.5 * info["nnz"]
+    g = torch.Generator(device="cuda")
+    g.manual_seed(4)
+    x = torch.randn(S.dim, dtype=torch.complex128, device="cuda", generator=g)
+    want = torch.empty_like(x)
+    U.matvec(x, want)
+    torch.cuda.synchronize()
+    st = torch.cuda.Stream()
+    for limit in (budget, 0):
+        for _ in range(4):
+            y = torch.zeros_like(x)
+            torch.cuda.synchronize()
+            B = D.Csr(S, S, P, max_bytes=limit)
+            B.matvec(x, y, stream=st)
+            st.synchronize()
+            assert torch.equal(torch.view_as_real(y).view(torch.int64), torch.view_as_real(want).view(torch.int64))
+            if limit and name != "projected":
+                assert B.info()["bytes"] < info["bytes"]
+            B.close()
