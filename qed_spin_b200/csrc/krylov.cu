@@ -815,15 +815,16 @@ void launch_pack(const std::vector<int>& set, const qb_sector* const* secs, cons
     const int cpl = (k + 7) / 8;
     auto go = [&](auto kernel) {
         set_smem(kernel, smem);
-        int dev = 0, sms = 148, per_sm = 1;
+        int dev = 0, sms = 148, per_sm = 0;
         cuda_check(cudaGetDevice(&dev), "device");
         cuda_check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "SM count");
         cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kPackThreads, smem), "occupancy");
+        if (per_sm < 1) throw Error(QB_ECUDA, "ftlm_pack: a block does not fit an SM");
         // at most two blocks per SM, and at most 2 GB of scratch in all (each block's results are its own,
         // whatever the grid)
         const std::size_t by_bytes = std::max<std::size_t>(1, (std::size_t(2) << 30) / slot.bytes);
         const int grid = static_cast<int>(std::min({set.size(), static_cast<std::size_t>(sms) *
-                                                                    std::max(1, std::min(per_sm, 2)), by_bytes}));
+                                                                    std::min(per_sm, 2), by_bytes}));
         d_items.alloc(items.size());
         counter.alloc(1);
         scratch.alloc(slot.bytes * grid);

@@ -155,3 +155,37 @@ def test_packed_blocks_equal_per_block_path(monkeypatch, dtype, tol):
     for key in ("lnZ", "E", "V"):
         a, b = out["4096"][key], out["0"][key]
         np.testing.assert_allclose(a, b, rtol=tol, atol=tol * np.abs(b).max(), err_msg=key)
+
+
+def _tables_model(name):
+    """Models whose packed blocks stage 13 to 49 KB of tables and program beside the kernel's own shared arrays."""
+    if name in ("6x4", "6x6"):
+        Lx, Ly, up = (6, 4, 4) if name == "6x4" else (6, 6, 3)
+        nn, nnn = lat.square_j1j2_bonds(Lx, Ly)
+        prods = ops.heisenberg_products(nn) + ops.heisenberg_products(nnn, 0.5)
+        specs = [lat.square_k0_sector(Lx, Ly, u) for u in (up, up - 1)]
+        return Lx * Ly, prods, specs
+    n = int(name.split("-")[1])
+    prods = ops.xxz_products(lat.chain_bonds(n), 1.0, 0.5) + ops.zeeman_z_products(n, 0.1)
+    if name.startswith("chiral"):
+        prods = prods + ops.chiral_products([(i, (i + 1) % n, (i + 2) % n) for i in range(n)], 0.2)
+    return n, prods, [lat.chain_sector(n, 4, 0), lat.chain_sector(n, 3, 5)]
+
+
+@pytest.mark.parametrize("dtype,tol", [("c128", 1e-10), ("c64", 1e-5)])
+@pytest.mark.parametrize("name", ["6x4", "6x6", "chiral-24", "field-24", "field-25", "field-27", "field-28"])
+def test_packed_blocks_of_models_with_large_tables(monkeypatch, name, dtype, tol):
+    """Packed and per-block curves agree (1e-10 relative in FP64 storage, 1e-5 in FP32: they differ in the order of
+    their inner-product sums) whatever the block's tables take of the shared memory."""
+    from qed_spin_b200 import device as D
+    n, prods, specs = _tables_model(name)
+    P = D.Program(ops.row_program(ops.from_products(n, prods)))
+    secs = [D.Sector(s) for s in specs]
+    assert all(s.dim <= 4096 for s in secs)
+    out = {}
+    for pack in ("4096", "0"):
+        monkeypatch.setenv("QB_FTLM_PACK_DIM", pack)
+        out[pack] = D.ftlm_blocks(secs, P, 12, 40, SEED, BETAS, dtype=dtype)
+    for key in ("lnZ", "E", "V"):
+        a, b = out["4096"][key], out["0"][key]
+        np.testing.assert_allclose(a, b, rtol=tol, atol=tol * np.abs(b).max(), err_msg=key)
