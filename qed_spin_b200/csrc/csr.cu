@@ -179,7 +179,7 @@ constexpr int kBuildWarps = 8;
 constexpr int kColSetBits = 8;   // the count pass's per-warp column set: 256 slots, for rows of up to 128 entries
 constexpr int kColSet = 1 << kColSetBits;
 
-template <class ST, bool kSame>
+template <class ST, bool kSame, int kCand>
 __global__ void __launch_bounds__(32 * kBuildWarps) csr_pass(DSector row, DSector col, DProgram P, bool prog_in_smem,
                                                              std::size_t stage_bytes, int pass,
                                                              unsigned long long* counts,
@@ -246,7 +246,7 @@ __global__ void __launch_bounds__(32 * kBuildWarps) csr_pass(DSector row, DSecto
                 if (vi >= 0) {
                     const cplx h = subgroup_value<ST>(sp.P, s, vi);
                     const ST t = s ^ static_cast<ST>(sp.P.group_flip[g]);
-                    ok = entry<kSame, ST>(col, sp.T, s, static_cast<long long>(r), w, t, h, j, c);
+                    ok = entry<kSame, ST, kCand>(col, sp.T, s, static_cast<long long>(r), w, t, h, j, c);
                 }
             }
             const unsigned bal = __ballot_sync(0xffffffffu, ok);
@@ -501,7 +501,7 @@ __global__ void __launch_bounds__(256) k_acting_total(DSector row, DSector col, 
 }
 
 // Rows lo .. lo + n of the walk into the slab, each row's entries in group order. walk_rows's loop and occupancy.
-template <class ST, bool kSame>
+template <class ST, bool kSame, int kCand>
 __global__ void __launch_bounds__(256, sizeof(ST) == 4 ? 6 : 5) k_slab_walk(DSector row, DSector col, DProgram P,
                                                                             bool prog_in_smem, u64 lo, u64 n,
                                                                             SlabEntries E) {
@@ -538,7 +538,7 @@ __global__ void __launch_bounds__(256, sizeof(ST) == 4 ? 6 : 5) k_slab_walk(DSec
             const ST t = s ^ static_cast<ST>(sp.P.group_flip[g]);
             long long j;
             cplx c;
-            if (!entry<kSame, ST>(col, sp.T, s, static_cast<long long>(r), w, t, h, j, c)) continue;
+            if (!entry<kSame, ST, kCand>(col, sp.T, s, static_cast<long long>(r), w, t, h, j, c)) continue;
             E.col[base + m] = static_cast<u32>(j);
             E.val[base + m] = make_double2(c.re, c.im);
             ++m;
@@ -949,12 +949,12 @@ void spmv_launch(const qb_csr* A, const void* in, void* out, int k, cudaStream_t
     cuda_check(cudaGetLastError(), "CSR matvec launch");
 }
 
-template <class ST, bool kSame>
+template <class ST, bool kSame, int kCand>
 void run_pass(const qb_sector* row, const qb_sector* col, const qb_program* P, int pass, unsigned long long* counts,
               const unsigned long long* row_ptr, u32* col_out, unsigned char* ids, int id_bytes, double2* full,
               const Dict& D, int* too_long) {
     bool in_smem = false;
-    const std::size_t stage_bytes = (smem_for(P, col, in_smem) + 15) & ~std::size_t(15);
+    const std::size_t stage_bytes = (smem_for(P, col, in_smem, kCand == kRowPairs) + 15) & ~std::size_t(15);
     // a row holds at most one entry per group: buffers of the program's groups rounded up to 32 (256 at most), so
     // more warps fit an SM than with 256-entry buffers
     const u32 ng = P->view.n_groups;
@@ -962,7 +962,7 @@ void run_pass(const qb_sector* row, const qb_sector* col, const qb_program* P, i
                                                           : kMaxRowEntries;
     const std::size_t smem = stage_bytes + static_cast<std::size_t>(kBuildWarps) * cap * (8 + 16) +
                              static_cast<std::size_t>(kBuildWarps) * kColSet * 8;
-    auto k = csr_pass<ST, kSame>;
+    auto k = csr_pass<ST, kSame, kCand>;
     set_smem(k, smem);
     int sms = 148, dev = 0;
     cudaGetDevice(&dev);
@@ -971,8 +971,8 @@ void run_pass(const qb_sector* row, const qb_sector* col, const qb_program* P, i
     const unsigned blocks = static_cast<unsigned>(std::max<u64>(1, std::min<u64>(want, static_cast<u64>(sms) * 16)));
     // row tags hold the low 32 bits of the row: rows past 2^32 take the sorting path
     const bool tag_rows = row->dim < (1ULL << 32);
-    k<<<blocks, 32 * kBuildWarps, smem>>>(row->view(), col->view(), P->view, in_smem, stage_bytes, pass, counts,
-                                          row_ptr, col_out, ids, id_bytes, full, D, too_long, tag_rows, cap);
+    k<<<blocks, 32 * kBuildWarps, smem>>>(row->view(), col->view(kCand == kRowPairs), P->view, in_smem, stage_bytes, pass,
+                                          counts, row_ptr, col_out, ids, id_bytes, full, D, too_long, tag_rows, cap);
     cuda_check(cudaGetLastError(), "CSR build pass");
 }
 
@@ -980,10 +980,10 @@ template <class ST>
 void build_passes(const qb_sector* row, const qb_sector* col, const qb_program* P, int pass, unsigned long long* counts,
                   const unsigned long long* row_ptr, u32* col_out, unsigned char* ids, int id_bytes, double2* full,
                   const Dict& D, int* too_long) {
-    if (row == col)
-        run_pass<ST, true>(row, col, P, pass, counts, row_ptr, col_out, ids, id_bytes, full, D, too_long);
-    else
-        run_pass<ST, false>(row, col, P, pass, counts, row_ptr, col_out, ids, id_bytes, full, D, too_long);
+    auto run = [&](auto go) { go(row, col, P, pass, counts, row_ptr, col_out, ids, id_bytes, full, D, too_long); };
+    if constexpr (sizeof(ST) == 8)
+        if (col->pair.p) return run(row == col ? run_pass<ST, true, kRowPairs> : run_pass<ST, false, kRowPairs>);
+    run(row == col ? run_pass<ST, true, kLists> : run_pass<ST, false, kLists>);
 }
 
 struct BitsHash {
@@ -1074,8 +1074,15 @@ bool build_slabs(const qb_sector* row, const qb_sector* col, const qb_program* P
     const u64 dim = row->dim;
     const int cap = static_cast<int>(P->view.n_groups);
     if (dim < kSlabMinRows || cap < 1 || cap > kMaxRowEntries) return false;
+    auto walk = row == col ? k_slab_walk<ST, true, kLists> : k_slab_walk<ST, false, kLists>;
+    bool pairs = false;
+    if constexpr (sizeof(ST) == 8)
+        if (col->pair.p) {
+            pairs = true;
+            walk = row == col ? k_slab_walk<ST, true, kRowPairs> : k_slab_walk<ST, false, kRowPairs>;
+        }
     bool in_smem = false;
-    const std::size_t smem = smem_for(P, col, in_smem);
+    const std::size_t smem = smem_for(P, col, in_smem, pairs);
     int sms = 148, dev = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -1084,7 +1091,7 @@ bool build_slabs(const qb_sector* row, const qb_sector* col, const qb_program* P
         cuda_check(cudaMemsetAsync(total.p, 0, 8, nullptr), "CSR clear");
         set_smem(k_acting_total<ST>, smem);
         const unsigned tb = static_cast<unsigned>(std::min<u64>((dim + 255) / 256, static_cast<u64>(sms) * 8));
-        k_acting_total<ST><<<tb, 256, smem>>>(row->view(), col->view(), P->view, in_smem, total.p);
+        k_acting_total<ST><<<tb, 256, smem>>>(row->view(), col->view(pairs), P->view, in_smem, total.p);
         cuda_check(cudaGetLastError(), "CSR bound");
         u64 most = 0;
         cuda_check(cudaMemcpy(&most, total.p, 8, cudaMemcpyDeviceToHost), "CSR bound");
@@ -1119,11 +1126,10 @@ bool build_slabs(const qb_sector* row, const qb_sector* col, const qb_program* P
         const SlabSet D{keys.p, kids.p, dict.p, reinterpret_cast<u32*>(flags.p), flags.p + 1};
         const std::size_t msmem = static_cast<std::size_t>(8) * 2 * cap * 8 + kNearBytes;
         int hflags[2] = {0, 0};
-        auto walk = row == col ? k_slab_walk<ST, true> : k_slab_walk<ST, false>;
         set_smem(walk, smem);
         for (u64 lo = 0; lo < dim; lo += chunk) {
             const u64 n = std::min(chunk, dim - lo);
-            walk<<<static_cast<unsigned>((n + 255) / 256), 256, smem>>>(row->view(), col->view(), P->view, in_smem, lo, n, E);
+            walk<<<static_cast<unsigned>((n + 255) / 256), 256, smem>>>(row->view(), col->view(pairs), P->view, in_smem, lo, n, E);
             cuda_check(cudaGetLastError(), "CSR slab walk");
             const unsigned blocks = static_cast<unsigned>(std::min<u64>((n + 7) / 8, static_cast<u64>(sms) * 8));
             slab_merge((cap + 31) / 32, blocks, msmem, n, E, counts.p, D);

@@ -34,11 +34,13 @@
 
 namespace qb {
 
-// team32.cu, team64.cu
+// team32.cu, team64.cu, team64_pairs.cu
 void launch_walk_team32(int shape, bool in32, bool out32, const qb_sector* row, const qb_sector* col, const qb_program* P,
                         const void* in, void* out, int k, cudaStream_t st);
 void launch_walk_team64(int shape, bool in32, bool out32, const qb_sector* row, const qb_sector* col, const qb_program* P,
                         const void* in, void* out, int k, cudaStream_t st);
+void launch_walk_team64_pairs(int shape, bool in32, bool out32, const qb_sector* row, const qb_sector* col,
+                              const qb_program* P, const void* in, void* out, int k, cudaStream_t st);
 
 namespace {
 
@@ -56,7 +58,7 @@ template <int NV> struct VecPtrs {
 // One thread per row. The row's groups are tested 32 at a time by every lane together (a converged
 // pass that builds the bitmask of the groups acting on the lane's row); the lanes then walk their own
 // acting groups in ascending order -- the diagonal first -- canonicalising one target each per step.
-template <int NV, class ST, bool kInF32, bool kOutF32, bool kSame>
+template <int NV, class ST, bool kInF32, bool kOutF32, bool kSame, int kCand>
 __global__ void __launch_bounds__(256, (NV <= 2 ? (sizeof(ST) == 4 ? 6 : 5) : 4)) walk_rows(DSector row, DSector col, DProgram P, bool prog_in_smem,
                                                     VecPtrs<NV> io) {
     extern __shared__ __align__(16) unsigned char smem[];
@@ -94,7 +96,7 @@ __global__ void __launch_bounds__(256, (NV <= 2 ? (sizeof(ST) == 4 ? 6 : 5) : 4)
             const ST t = s ^ static_cast<ST>(sp.P.group_flip[g]);
             long long j;
             cplx c;
-            if (!entry<kSame, ST, sizeof(ST) == 4>(col, sp.T, s, static_cast<long long>(r), w, t, h, j, c)) continue;
+            if (!entry<kSame, ST, kCand>(col, sp.T, s, static_cast<long long>(r), w, t, h, j, c)) continue;
 #pragma unroll
             for (int v = 0; v < NV; ++v)
                 acc[v] = cadd(acc[v], cmul(c, St::load(static_cast<const typename St::T*>(io.in[v]), static_cast<std::size_t>(j))));
@@ -118,7 +120,7 @@ struct WarpSlots {
     int ok[32];
 };
 
-template <int NV, class ST, bool kInF32, bool kOutF32, bool kSame>
+template <int NV, class ST, bool kInF32, bool kOutF32, bool kSame, int kCand>
 __global__ void __launch_bounds__(256, 4) walk_warp(DSector row, DSector col, DProgram P, bool prog_in_smem,
                                                     std::size_t stage_bytes, VecPtrs<NV> io) {
     extern __shared__ __align__(16) unsigned char smem[];
@@ -184,7 +186,7 @@ __global__ void __launch_bounds__(256, 4) walk_warp(DSector row, DSector col, DP
                 const ST t = so ^ static_cast<ST>(sp.P.group_flip[g]);
                 long long j;
                 cplx c;
-                if (entry<kSame, ST>(col, sp.T, so, static_cast<long long>(r0 + o), W.w[o], t, h, j, c)) {
+                if (entry<kSame, ST, kCand>(col, sp.T, so, static_cast<long long>(r0 + o), W.w[o], t, h, j, c)) {
                     ok = 1;
 #pragma unroll
                     for (int v = 0; v < NV; ++v) {
@@ -219,6 +221,8 @@ void launch_team_st(int shape, bool in32, bool out32, const qb_sector* row, cons
                     const void* in, void* out, int k, cudaStream_t st) {
     if (sizeof(ST) == 4)
         launch_walk_team32(shape, in32, out32, row, col, P, in, out, k, st);
+    else if (col->pair.p)
+        launch_walk_team64_pairs(shape, in32, out32, row, col, P, in, out, k, st);
     else
         launch_walk_team64(shape, in32, out32, row, col, P, in, out, k, st);
 }
@@ -260,23 +264,39 @@ std::string walk_key(const qb_sector* row, const qb_sector* col, const qb_progra
            (row == col ? ".same" : ".cross");
 }
 
+// kRows, kWarp: the candidates' form for walk_rows and for walk_warp.
+template <int NV, class ST, bool kF32, bool kOutF32, bool kSame, int kRows, int kWarp>
+void launch_rows_cand(int shape, const qb_sector* row, const qb_sector* col, const qb_program* P,
+                      const VecPtrs<NV>& io, cudaStream_t st) {
+    constexpr bool kPairs = kRows == kRowPairs;
+    bool in_smem = false;
+    const std::size_t stage = (smem_for(P, col, in_smem, kPairs) + 15) & ~std::size_t(15);
+    const unsigned blocks = static_cast<unsigned>((row->dim + 255) / 256);
+    if (shape == 0) {
+        auto k = walk_rows<NV, ST, kF32, kOutF32, kSame, kRows>;
+        set_smem(k, stage);
+        k<<<blocks, 256, stage, st>>>(row->view(), col->view(kPairs), P->view, in_smem, io);
+    } else {
+        auto k = walk_warp<NV, ST, kF32, kOutF32, kSame, kWarp>;
+        const std::size_t smem = stage + 8 * (sizeof(WarpSlots) + 32 * NV * sizeof(double2));
+        set_smem(k, smem);
+        k<<<blocks, 256, smem, st>>>(row->view(), col->view(kPairs), P->view, in_smem, stage, io);
+    }
+    cuda_check(cudaGetLastError(), "walk launch");
+}
+
+// 64-bit states: row pairs where the sector has their table, else lists. 32-bit states: masks, a warp's states lists.
 template <int NV, class ST, bool kF32, bool kOutF32, bool kSame>
 void launch_rows_shape(int shape, const qb_sector* row, const qb_sector* col, const qb_program* P,
                        const VecPtrs<NV>& io, cudaStream_t st) {
-    bool in_smem = false;
-    const std::size_t stage = (smem_for(P, col, in_smem) + 15) & ~std::size_t(15);
-    const unsigned blocks = static_cast<unsigned>((row->dim + 255) / 256);
-    if (shape == 0) {
-        auto k = walk_rows<NV, ST, kF32, kOutF32, kSame>;
-        set_smem(k, stage);
-        k<<<blocks, 256, stage, st>>>(row->view(), col->view(), P->view, in_smem, io);
+    if constexpr (sizeof(ST) == 4) {
+        launch_rows_cand<NV, ST, kF32, kOutF32, kSame, kMasks, kLists>(shape, row, col, P, io, st);
     } else {
-        auto k = walk_warp<NV, ST, kF32, kOutF32, kSame>;
-        const std::size_t smem = stage + 8 * (sizeof(WarpSlots) + 32 * NV * sizeof(double2));
-        set_smem(k, smem);
-        k<<<blocks, 256, smem, st>>>(row->view(), col->view(), P->view, in_smem, stage, io);
+        if (col->pair.p)
+            launch_rows_cand<NV, ST, kF32, kOutF32, kSame, kRowPairs, kRowPairs>(shape, row, col, P, io, st);
+        else
+            launch_rows_cand<NV, ST, kF32, kOutF32, kSame, kLists, kLists>(shape, row, col, P, io, st);
     }
-    cuda_check(cudaGetLastError(), "walk launch");
 }
 
 // The row walk over NV vectors, as the tuner picks: one thread per state (walk_rows), a warp's states compacted

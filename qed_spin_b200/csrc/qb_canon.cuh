@@ -196,6 +196,11 @@ template <class ST> struct BlockPattern {
     }
 };
 
+// How a kernel finds the elements that may bring a state to its representative. Each is a form of its own of a kernel, chosen
+// by the host: the row pairs' code beside the lists', behind a test of the sector, cost the 64-bit kernels of sectors that
+// have no pair table registers and spills (one vector in teams of four lanes, 34 sites, 158 k rows: 659 -> 855 us).
+enum Cand : int { kLists = 0, kMasks = 1, kRowPairs = 2 };
+
 // Torus rows: fn(g) in ascending order for the elements whose image has the least pair of leading rows, a subset of
 // for_each_candidate's that still holds every element of least key. Element a + Lx b rotates row b's bits by a and
 // brings it to row 0, row b + 1 behind it; the candidates are bits b Lx + a of one mask, read in order. The rows of a
@@ -332,14 +337,14 @@ __device__ __forceinline__ ST canonicalize_masked(const DSector& S, const Tables
 
 // Representative of t and the conjugated character sum over the elements that reach it.
 // With a key order the images are compared in place (key_below), so no image is mapped to its key.
-template <class ST, bool kMasked = false>
+template <class ST, int kCand = kLists>
 __device__ __forceinline__ ST canonicalize(const DSector& S, const Tables& T, ST t, double& acc_re, double& acc_im) {
     ST rb = static_cast<ST>(~static_cast<ST>(0));
     acc_re = 0.0;
     acc_im = 0.0;
-    if constexpr (kMasked)
+    if constexpr (kCand == kMasks)
         if (S.slc.on) return canonicalize_masked<ST>(S, T, t, acc_re, acc_im);
-    if (!kMasked && S.slc.on) {
+    if (kCand == kRowPairs || (kCand == kLists && S.slc.on)) {
         bool have = false;
         auto visit = [&](int g) {
             const ST img = apply_elem<ST>(S, T, t, g);
@@ -355,7 +360,7 @@ __device__ __forceinline__ ST canonicalize(const DSector& S, const Tables& T, ST
                 acc_im = __dsub_rn(acc_im, c.y);
             }
         };
-        if (sizeof(ST) == 8 && T.pair)
+        if constexpr (kCand == kRowPairs)
             for_each_row_candidate<ST>(S, T.pair, t, visit);
         else
             for_each_candidate(S, T.pack, BlockPattern<ST>(S, T.to_key, t), visit);
@@ -464,12 +469,12 @@ __device__ __forceinline__ long long index_of_rep(const DSector& S, u64 rb) {
 }
 
 // index_and_projection: index of t's orbit in S (or -1) and conj(beta_t) * inv_norm[index].
-template <class ST = u64, bool kMasked = false>
+template <class ST = u64, int kCand = kLists>
 __device__ __forceinline__ long long index_and_projection(const DSector& S, const Tables& T, ST t, double& pre,
                                                           double& pim) {
     if (__popcll(static_cast<u64>(t)) != S.n_up) return -1;
     double are, aim;
-    const u64 rb = static_cast<u64>(canonicalize<ST, kMasked>(S, T, t, are, aim));
+    const u64 rb = static_cast<u64>(canonicalize<ST, kCand>(S, T, t, are, aim));
     long long j;
     double s;
     if (S.lookup >= 3) {

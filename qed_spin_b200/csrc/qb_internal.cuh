@@ -142,7 +142,8 @@ struct DSlc {
     // block j is sites [jL, (j+1)L) in order: its pattern is state bits jL .. jL+L-1, no key needed
     int contig = 0;
     // torus translations of more than 32 sites whose blocks are the rows (build_pair_table): per pair of neighbouring rows, the least
-    // (first, second) row pattern over the row rotations << 8 | the rotations that reach it; null elsewhere
+    // (first, second) row pattern over the row rotations << 8 | the rotations that reach it; null elsewhere, and for
+    // kernels that do not read it
     const u32* pair = nullptr;      // 1 << 2L
 };
 
@@ -227,7 +228,8 @@ struct qb_sector {
     std::vector<std::uint64_t> desc_flips;
     int desc_slc_mode = 0, desc_lookup = 0;
     bool registered = false;          // owned by the registry (qb_sector_acquire / qb_sector_release)
-    qb::DSector view() const;
+    // pairs: with the row-pair table, for the kernels that read it (kRowPairs)
+    qb::DSector view(bool pairs = false) const;
     std::uint64_t device_bytes() const;
 };
 

@@ -1,6 +1,7 @@
 // =============================================================================
 // qb_team.cuh -- the team walk: a team of lanes per row, for blocks of vectors and for one vector on a small sector.
-// Compiled for 32-bit states (team32.cu) and 64-bit ones (team64.cu).
+// Compiled for 32-bit states (team32.cu), 64-bit ones (team64.cu) and 64-bit ones of sectors with row pairs
+// (team64_pairs.cu).
 // =============================================================================
 #pragma once
 
@@ -15,7 +16,7 @@ namespace {
 // the loads between. 32-bit states when every state fits, and registers for four blocks an SM when a lane owns several
 // columns: chain-24, 40 FP32 vectors 183 -> 165 us (177 at three blocks, 236 with the registers of one); one column
 // keeps the registers of one block, as a small sector fills few: chain-20, one vector 28.7 -> 25.1 us (28.7 at four).
-template <class State, int kTeam, int kCpl, bool kF32, bool kOutF32, bool kSame>
+template <class State, int kTeam, int kCpl, bool kF32, bool kOutF32, bool kSame, int kCand>
 __global__ void __launch_bounds__(256, kCpl == 1 ? 1 : 4) walk_team(DSector row, DSector col, DProgram P, bool prog_in_smem,
                                                  const void* in_v, void* out_v, int k) {
     extern __shared__ __align__(16) unsigned char smem[];
@@ -44,7 +45,7 @@ __global__ void __launch_bounds__(256, kCpl == 1 ? 1 : 4) walk_team(DSector row,
         long long j = -1;
         cplx cv{0.0, 0.0};
         bool act = live && g < sp.P.n_groups && connection<State>(sp.P, s, g, t, h);
-        if (act) act = entry<kSame, State>(col, sp.T, s, static_cast<long long>(r), w, t, h, j, cv);
+        if (act) act = entry<kSame, State, kCand>(col, sp.T, s, static_cast<long long>(r), w, t, h, j, cv);
         unsigned acting = __ballot_sync(0xffffffffu, act) & team_mask;
         while (acting) {
             const int src = __ffs(acting) - 1;
@@ -64,66 +65,66 @@ __global__ void __launch_bounds__(256, kCpl == 1 ? 1 : 4) walk_team(DSector row,
         if (c0 + c < k) So::store(out, static_cast<std::size_t>(r) * k + c0 + c, acc[c]);
 }
 
-template <class State, int kTeam, int kCpl, bool kF32, bool kOutF32>
+template <class State, int kCand, int kTeam, int kCpl, bool kF32, bool kOutF32>
 void team_launch(const qb_sector* row, const qb_sector* col, const qb_program* P, const void* in, void* out, int k,
                  cudaStream_t st) {
     bool in_smem = false;
-    const std::size_t smem = smem_for(P, col, in_smem);
+    const std::size_t smem = smem_for(P, col, in_smem, kCand == kRowPairs);
     constexpr int kRowsPerWarp = 32 / kTeam;
     const std::uint64_t warps = (row->dim + kRowsPerWarp - 1) / kRowsPerWarp;
     const unsigned blocks = static_cast<unsigned>((warps * 32 + 255) / 256);
     auto go = [&](auto kk) {
         set_smem(kk, smem);
-        kk<<<blocks, 256, smem, st>>>(row->view(), col->view(), P->view, in_smem, in, out, k);
+        kk<<<blocks, 256, smem, st>>>(row->view(), col->view(kCand == kRowPairs), P->view, in_smem, in, out, k);
     };
     if (row == col)
-        go(walk_team<State, kTeam, kCpl, kF32, kOutF32, true>);
+        go(walk_team<State, kTeam, kCpl, kF32, kOutF32, true, kCand>);
     else
-        go(walk_team<State, kTeam, kCpl, kF32, kOutF32, false>);
+        go(walk_team<State, kTeam, kCpl, kF32, kOutF32, false, kCand>);
     cuda_check(cudaGetLastError(), "walk_team launch");
 }
 
 // The columns per lane: the least of 1, 2, 4, 5 and 8 that covers k; a team that covers the 64 vectors of a block walk
 // with fewer has no kernel of the larger ones.
-template <class State, int kTeam, bool kF32, bool kOutF32>
+template <class State, int kCand, int kTeam, bool kF32, bool kOutF32>
 void team_cols(const qb_sector* row, const qb_sector* col, const qb_program* P, const void* in, void* out, int k,
                cudaStream_t st) {
     const int cpl = (k + kTeam - 1) / kTeam;
-    if (cpl <= 1) return team_launch<State, kTeam, 1, kF32, kOutF32>(row, col, P, in, out, k, st);
-    if (cpl <= 2) return team_launch<State, kTeam, 2, kF32, kOutF32>(row, col, P, in, out, k, st);
+    if (cpl <= 1) return team_launch<State, kCand, kTeam, 1, kF32, kOutF32>(row, col, P, in, out, k, st);
+    if (cpl <= 2) return team_launch<State, kCand, kTeam, 2, kF32, kOutF32>(row, col, P, in, out, k, st);
     if constexpr (kTeam < 32)
-        if (cpl <= 4) return team_launch<State, kTeam, 4, kF32, kOutF32>(row, col, P, in, out, k, st);
+        if (cpl <= 4) return team_launch<State, kCand, kTeam, 4, kF32, kOutF32>(row, col, P, in, out, k, st);
     if constexpr (kTeam < 16) {
-        if (cpl <= 5) return team_launch<State, kTeam, 5, kF32, kOutF32>(row, col, P, in, out, k, st);
-        if (cpl <= 8) return team_launch<State, kTeam, 8, kF32, kOutF32>(row, col, P, in, out, k, st);
+        if (cpl <= 5) return team_launch<State, kCand, kTeam, 5, kF32, kOutF32>(row, col, P, in, out, k, st);
+        if (cpl <= 8) return team_launch<State, kCand, kTeam, 8, kF32, kOutF32>(row, col, P, in, out, k, st);
     }
     throw Error(QB_EUNSUPPORTED, "block matvec: at most 64 vectors");
 }
 
-template <class State, bool kF32, bool kOutF32>
+template <class State, int kCand, bool kF32, bool kOutF32>
 void team_shape(int shape, const qb_sector* row, const qb_sector* col, const qb_program* P, const void* in, void* out,
                 int k, cudaStream_t st) {
     if (shape == 0)
-        team_cols<State, 8, kF32, kOutF32>(row, col, P, in, out, k, st);
+        team_cols<State, kCand, 8, kF32, kOutF32>(row, col, P, in, out, k, st);
     else if (shape == 1)
-        team_cols<State, 16, kF32, kOutF32>(row, col, P, in, out, k, st);
+        team_cols<State, kCand, 16, kF32, kOutF32>(row, col, P, in, out, k, st);
     else if (shape == 2)
-        team_cols<State, 32, kF32, kOutF32>(row, col, P, in, out, k, st);
+        team_cols<State, kCand, 32, kF32, kOutF32>(row, col, P, in, out, k, st);
     else
-        team_cols<State, 4, kF32, kOutF32>(row, col, P, in, out, k, st);
+        team_cols<State, kCand, 4, kF32, kOutF32>(row, col, P, in, out, k, st);
 }
 
-template <class State>
+template <class State, int kCand>
 void launch_walk_team(int shape, bool in32, bool out32, const qb_sector* row, const qb_sector* col, const qb_program* P,
                       const void* in, void* out, int k, cudaStream_t st) {
     if (in32 && out32)
-        team_shape<State, true, true>(shape, row, col, P, in, out, k, st);
+        team_shape<State, kCand, true, true>(shape, row, col, P, in, out, k, st);
     else if (in32)
-        team_shape<State, true, false>(shape, row, col, P, in, out, k, st);
+        team_shape<State, kCand, true, false>(shape, row, col, P, in, out, k, st);
     else if (out32)
-        team_shape<State, false, true>(shape, row, col, P, in, out, k, st);
+        team_shape<State, kCand, false, true>(shape, row, col, P, in, out, k, st);
     else
-        team_shape<State, false, false>(shape, row, col, P, in, out, k, st);
+        team_shape<State, kCand, false, false>(shape, row, col, P, in, out, k, st);
 }
 
 }  // namespace

@@ -102,7 +102,7 @@ template <class ST> __device__ __forceinline__ bool connection(const DProgram& P
 }
 
 // The entry of one connection: column j and value c, or false when the target's orbit cancels.
-template <bool kSame, class ST, bool kMasked = false>
+template <bool kSame, class ST, int kCand = kLists>
 __device__ __forceinline__ bool entry(const DSector& col, const Tables& T, ST s, long long r, double w, ST t,
                                       cplx h, long long& j, cplx& c) {
     if (kSame && t == s) {
@@ -111,7 +111,7 @@ __device__ __forceinline__ bool entry(const DSector& col, const Tables& T, ST s,
         return true;
     }
     double pre, pim;
-    j = index_and_projection<ST, kMasked>(col, T, t, pre, pim);
+    j = index_and_projection<ST, kCand>(col, T, t, pre, pim);
     if (j < 0) return false;
     c = rscale(w, cconj(cmul(h, {pre, pim})));
     return true;
@@ -136,8 +136,9 @@ template <> struct Store<true> {
 };
 
 
-inline std::size_t smem_for(const qb_program* P, const qb_sector* col, bool& in_smem) {
-    const std::size_t tables = (tables_smem_bytes(col->view()) + 15) & ~std::size_t(15);
+// pairs: for a kernel of the row-pair form.
+inline std::size_t smem_for(const qb_program* P, const qb_sector* col, bool& in_smem, bool pairs = false) {
+    const std::size_t tables = (tables_smem_bytes(col->view(pairs)) + 15) & ~std::size_t(15);
     in_smem = P->view.smem_bytes <= 40 * 1024;
     return tables + (in_smem ? P->view.smem_bytes : 0);
 }

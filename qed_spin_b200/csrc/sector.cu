@@ -737,7 +737,7 @@ void build_lookup(qb_sector& s, int want) {
 }  // namespace
 }  // namespace qb
 
-qb::DSector qb_sector::view() const {
+qb::DSector qb_sector::view(bool pairs) const {
     qb::DSector v;
     v.N = N;
     v.n_up = n_up;
@@ -760,7 +760,7 @@ qb::DSector qb_sector::view() const {
     v.slc.to_key = to_key.p;
     v.slc.pack = lead_pack.p;
     v.slc.cand = cand.p;
-    v.slc.pair = pair.p;
+    v.slc.pair = pairs ? pair.p : nullptr;
     v.gkind = gkind;
     v.Lx = Lx;
     v.edesc = edesc.p;
