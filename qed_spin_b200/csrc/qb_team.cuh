@@ -13,12 +13,18 @@ namespace {
 // Team kernel: kTeam lanes per row (4, 8, 16 or 32), kCpl columns per lane (k <= kTeam kCpl vectors). Every column
 // adds its row's entries in group order whatever kTeam is, so the team size changes only the time.
 // What bounds it: instruction issue (canonicalisation, then eight FP64 operations an element and target) and the latency of
-// the loads between. 32-bit states when every state fits, and registers for four blocks an SM when a lane owns several
-// columns: chain-24, 40 FP32 vectors 183 -> 165 us (177 at three blocks, 236 with the registers of one); one column
-// keeps the registers of one block, as a small sector fills few: chain-20, one vector 28.7 -> 25.1 us (28.7 at four).
+// the loads between. 32-bit states when every state fits. Registers: the compiler's own count (60 to 64 for up to five
+// columns of 32-bit states) with no bound on the blocks an SM. A bound of one block an SM gave one column 128 registers:
+// 2% faster on the 9,252 rows of chain-20 alone (25.0 against 25.6 us), 1.2 to 1.7x slower from 20 k rows, where a launch is
+// more than two blocks an SM (one vector, chain-24 at 8 spins up 52.8 against 39.0 us; 6x5 at 7 spins up 400 against 274).
+// A bound of four blocks spills in 64-bit states (one vector, 36 sites at 5 spins up 69.7 against 64.3 us) and from five
+// columns on (chain-24, 40 FP64 vectors 203 against 188 us, FP32 159 against 155). Two columns of 32-bit states in teams of 32
+// are the exception: there the compiler's count spills (64 FP64 vectors, chiral-24 at 9 spins up 248 against 232 us).
+template <class State, int kTeam, int kCpl>
+constexpr int kTeamBlocks = sizeof(State) == 4 && kTeam == 32 && kCpl == 2 ? 4 : 0;   // 0: no bound
 template <class State, int kTeam, int kCpl, bool kF32, bool kOutF32, bool kSame, int kCand>
-__global__ void __launch_bounds__(256, kCpl == 1 ? 1 : 4) walk_team(DSector row, DSector col, DProgram P, bool prog_in_smem,
-                                                 const void* in_v, void* out_v, int k) {
+__global__ void __launch_bounds__(256, kTeamBlocks<State, kTeam, kCpl>) walk_team(DSector row, DSector col, DProgram P,
+                                                 bool prog_in_smem, const void* in_v, void* out_v, int k) {
     extern __shared__ __align__(16) unsigned char smem[];
     using St = Store<kF32>;
     using So = Store<kOutF32>;
