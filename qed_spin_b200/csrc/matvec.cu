@@ -285,12 +285,20 @@ void launch_rows_cand(int shape, const qb_sector* row, const qb_sector* col, con
     cuda_check(cudaGetLastError(), "walk launch");
 }
 
-// 64-bit states: row pairs where the sector has their table, else lists. 32-bit states: masks, a warp's states lists.
+// 64-bit states: row pairs where the sector has their table, else lists. 32-bit states: masks, or lists where the key order
+// has two blocks, or three and characters +1 and -1: few blocks rarely tie, and then a block's list is one element, read
+// as it is found. Lists against masks, one vector, us: two blocks chain-26 179 / 198, chain-28 565 / 610, 6x5 at 7 spins up
+// 374 / 432; three blocks chain-27 360 / 378 at k = 0 and 404 / 379 at k = 1; five chiral-25 434 / 361, 5x5 876 / 807; no
+// key order chain-23 136 / 125, chain-29 1,941 / 1,753. A warp's states (walk_warp) keep lists.
 template <int NV, class ST, bool kF32, bool kOutF32, bool kSame>
 void launch_rows_shape(int shape, const qb_sector* row, const qb_sector* col, const qb_program* P,
                        const VecPtrs<NV>& io, cudaStream_t st) {
     if constexpr (sizeof(ST) == 4) {
-        launch_rows_cand<NV, ST, kF32, kOutF32, kSame, kMasks, kLists>(shape, row, col, P, io, st);
+        const DSector c = col->view();
+        if (c.slc.on && (c.slc.m == 2 || (c.slc.m == 3 && c.unit_chars)))
+            launch_rows_cand<NV, ST, kF32, kOutF32, kSame, kLists, kLists>(shape, row, col, P, io, st);
+        else
+            launch_rows_cand<NV, ST, kF32, kOutF32, kSame, kMasks, kLists>(shape, row, col, P, io, st);
     } else {
         if (col->pair.p)
             launch_rows_cand<NV, ST, kF32, kOutF32, kSame, kRowPairs, kRowPairs>(shape, row, col, P, io, st);

@@ -305,8 +305,9 @@ __device__ __forceinline__ int next_candidate(const DSector& S, const Tables& T,
 // canonicalize for the thread-per-row walk of 32-bit states, with a key order: the candidates are collected as a mask and
 // visited in ascending order by one loop, a single copy of the image and its comparison whatever blocks tie and
 // whatever the characters are, where the lists (for_each_candidate) make five, and the merge of several keeps its
-// cursors in local memory. chiral-27 at a complex momentum 748 -> 705 us; the team walk and the 64-bit states stay with
-// the lists (chain-24's block walk 166 against 171 us, 6x6 66.0 against 66.6 ms).
+// cursors in local memory. chiral-27 at a complex momentum 740 -> 700 us, chiral-25 434 -> 361; launch_rows_shape says
+// where lists are faster. The team walk and the 64-bit states stay with the lists (chain-24's block walk 166 against
+// 171 us, 6x6 66.0 against 66.6 ms).
 template <class ST>
 __device__ __forceinline__ ST canonicalize_masked(const DSector& S, const Tables& T, ST t, double& acc_re, double& acc_im) {
     KeyMin<ST> k{static_cast<ST>(~static_cast<ST>(0)), 0.0, 0.0, false};
