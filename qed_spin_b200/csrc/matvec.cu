@@ -227,24 +227,24 @@ void launch_team_st(int shape, bool in32, bool out32, const qb_sector* row, cons
         launch_walk_team64(shape, in32, out32, row, col, P, in, out, k, st);
 }
 
-// The calling thread's last shape choices by launch identity (the sectors, the program, a tag of the vectors),
-// so that a step does not rebuild its size-class key. An entry made under another tuner generation is ignored;
-// one left by a destroyed object whose address came back can only cost time, as every shape gives the same y.
+// The calling thread's last shape choices by launch identity (the sectors' and the program's serial numbers, a tag of the
+// vectors), so that a step does not rebuild its size-class key. An entry made under another tuner generation is ignored.
 struct ShapeMemo {
     struct Entry {
-        const void *row = nullptr, *col = nullptr, *prog = nullptr;
+        std::uint64_t row = 0, col = 0, prog = 0;
         int tag = -1, shape = 0;
         unsigned gen = 0;
     };
     Entry e[8];
     int next = 0;
-    int find(const void* r, const void* c, const void* p, int tag, unsigned gen) const {
+    int find(const qb_sector* r, const qb_sector* c, const qb_program* p, int tag, unsigned gen) const {
         for (const auto& x : e)
-            if (x.row == r && x.col == c && x.prog == p && x.tag == tag && x.gen == gen) return x.shape;
+            if (x.row == r->serial && x.col == c->serial && x.prog == p->serial && x.tag == tag && x.gen == gen)
+                return x.shape;
         return -1;
     }
-    void put(const void* r, const void* c, const void* p, int tag, unsigned gen, int shape) {
-        e[next] = Entry{r, c, p, tag, shape, gen};
+    void put(const qb_sector* r, const qb_sector* c, const qb_program* p, int tag, unsigned gen, int shape) {
+        e[next] = Entry{r->serial, c->serial, p->serial, tag, shape, gen};
         next = (next + 1) % 8;
     }
 };

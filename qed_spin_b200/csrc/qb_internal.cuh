@@ -19,6 +19,7 @@
 
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdint>
 #include <functional>
 #include <stdexcept>
@@ -197,8 +198,17 @@ struct DProgram {
 
 }  // namespace qb
 
+namespace qb {
+// A number of its own for every sector and program of the process (an address comes back when its object is destroyed).
+inline std::uint64_t next_serial() {
+    static std::atomic<std::uint64_t> n{0};
+    return ++n;
+}
+}  // namespace qb
+
 // The host objects behind the opaque handles.
 struct qb_sector {
+    const std::uint64_t serial = qb::next_serial();
     int N = 0, n_up = 0, G = 0, bpw = 0;
     std::uint64_t dim = 0;
     qb::DevBuf<qb::u64> reps;
@@ -236,6 +246,7 @@ struct qb_sector {
 struct qb_csr;
 
 struct qb_program {
+    const std::uint64_t serial = qb::next_serial();
     qb::DevBuf<unsigned char> blob;   // every array back to back (8-byte aligned), staged as one copy
     qb::DProgram view;
     double norm_bound = 0.0;          // sum of |coeff|

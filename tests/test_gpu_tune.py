@@ -142,3 +142,21 @@ def test_tuner_modes_and_cache():
     D.tune_mode(1)
     with pytest.raises(ValueError):
         D.tune_mode(7)
+
+
+def test_a_new_sector_does_not_inherit_a_destroyed_ones_shape():
+    """Sectors made and destroyed in turn, often at one address: each size class is timed for itself on first use."""
+    from qed_spin_b200 import device as D
+    n = 18
+    P = D.Program(ops.row_program(ops.from_products(n, ops.heisenberg_products(lat.chain_bonds(n), 1.0))))
+    D.tune_mode(1)
+    D.tune_clear()
+    seen = set()
+    for up in (9, 2, 7, 4, 3, 5):
+        S = D.Sector(lat.chain_sector(n, up, 1))
+        x = torch.ones(S.dim, dtype=torch.complex128, device="cuda")
+        D.matvec(S, S, P, [x], [torch.empty_like(x)])
+        seen.add((S.dim - 1).bit_length())
+        S.close()
+        del S
+    assert len(seen) == 6 and sum(k.startswith("walk|") for k in D.tune_entries()) == len(seen)
