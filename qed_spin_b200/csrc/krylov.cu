@@ -550,8 +550,11 @@ __host__ __device__ inline PackSlot pack_slot(std::uint64_t n_max, int max_entri
 }
 
 // Threads of a packed block's CTA: a CTA runs its whole block alone, so its own warps are all that hides its loads' latency
-// (a model of 34 packed blocks leaves 114 SMs idle as it is). The 34 sampled blocks of a 16-site chain, 715 to 810
-// states in FP64: 18.3 ms with 256 threads, 9.6 with 512.
+// (a model of 34 packed blocks leaves 114 SMs idle as it is), with all the registers of its SM: a bound of one block an SM
+// keeps the forms without spills, but for 8 bytes at 64 FP64 samples (unbounded, the compiler gave most FP32 forms 64
+// registers and 240 to 404 bytes of spills). A call on the 32 sampled blocks of a 16-site chain, up to 810 states, 40 samples, 60 steps: 14.8 ms with 256
+// threads, 9.2 with 512 in FP64; 13.2, 9.8 with the spills, 8.7 without in FP32. On 238 blocks of a 17-site chain, more
+// than the SMs, 44.2 -> 23.0 and 30.9 -> 17.0 ms.
 constexpr int kPackThreads = 512;
 constexpr int kPackGroups = kPackThreads / 8;   // row groups of 8 lanes
 
@@ -564,7 +567,7 @@ __device__ __forceinline__ double pack_col_sum(double (*red)[kPackGroups + 1], i
 }
 
 template <class T, class ST, int CPL>
-__global__ void __launch_bounds__(kPackThreads) ftlm_pack(const PackItem* items, int n_items, unsigned* next_item, int k,
+__global__ void __launch_bounds__(kPackThreads, 1) ftlm_pack(const PackItem* items, int n_items, unsigned* next_item, int k,
                                                  int max_entries, const double2* G_all, double* alpha,
                                                  double* beta, unsigned char* scratch, PackSlot slot) {
     using Rt = typename Work<T>::R;
