@@ -213,6 +213,7 @@ __device__ __forceinline__ bool grid_meet(const StepSync& S) {
         met = 1;
         __threadfence();
         const unsigned g = *static_cast<volatile unsigned*>(S.gen);
+        __threadfence();   // the generation is read before the arrival that may end it
         if (atomicAdd(S.count, 1u) == gridDim.x - 1) {
             *S.count = 0;
             __threadfence();
