@@ -15,6 +15,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <memory>
 #include <mutex>
 #include <numeric>
 
@@ -549,19 +550,36 @@ int classify_group(const int32_t* perms, int G, int N, int& Lx, std::vector<u64>
     return 0;
 }
 
-// A table copied in stream order: a pageable source is staged before the call returns, and the sector's creation ends
-// with a synchronisation, so a table needs none of its own (a dozen of them were a third of a small sector's creation).
-template <class T> void upload_queued(DevBuf<T>& b, const std::vector<T>& v) {
-    b.alloc(v.size());
-    if (!v.empty())
-        cuda_check(cudaMemcpyAsync(b.p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, cudaStreamPerThread), "upload");
-}
+// The tables of a sector in the making, copied in stream order: each is kept here until finish() has waited for the copies,
+// since nothing promises that a pageable source has been read when the call that queues its copy returns. One wait for
+// them all: with a synchronisation each, a dozen tables were a third of a small sector's creation.
+class QueuedUploads {
+public:
+    ~QueuedUploads() {
+        if (!held_.empty()) cudaStreamSynchronize(cudaStreamPerThread);   // left by an exception
+    }
+    template <class T> void add(DevBuf<T>& b, std::vector<T> v) {
+        b.alloc(v.size());
+        if (v.empty()) return;
+        const auto keep = std::make_shared<std::vector<T>>(std::move(v));
+        held_.push_back(keep);
+        cuda_check(cudaMemcpyAsync(b.p, keep->data(), keep->size() * sizeof(T), cudaMemcpyHostToDevice, cudaStreamPerThread),
+                   "upload");
+    }
+    void finish() {
+        cuda_check(cudaStreamSynchronize(cudaStreamPerThread), "sector");
+        held_.clear();
+    }
+
+private:
+    std::vector<std::shared_ptr<void>> held_;
+};
 
 // The row-pair table (for_each_row_candidate) when the group is every translation of a torus, numbered a + Lx b and
 // without flips, and the key order's blocks are its rows, of at most 6 sites (16 KB), with more than 32 sites (the
 // kernels of 32-bit states, chains above all, stay without the second kind of candidate): entry (first | second << L) holds
 // the least (rot_a first << L | rot_a second) over the rotations a, << 8, and the rotations that reach it.
-void build_pair_table(qb_sector& s, const qb_sector_desc& d) {
+void build_pair_table(qb_sector& s, const qb_sector_desc& d, QueuedUploads& up) {
     const int L = s.slc_L, m = s.slc_m;
     if (!s.slc_on || !s.slc_contig || s.gkind != 2 || s.Lx != L || L > 6 || s.G != L * m || s.N <= 32) return;
     for (int g = 0; g < s.G; ++g) {
@@ -580,17 +598,17 @@ void build_pair_table(qb_sector& s, const qb_sector_desc& d) {
         }
         t[p] = best << 8 | mask;
     }
-    upload_queued(s.pair, t);
+    up.add(s.pair, std::move(t));
 }
 
-void upload_group(qb_sector& s, const qb_sector_desc& d) {
+void upload_group(qb_sector& s, const qb_sector_desc& d, QueuedUploads& up) {
     const int G = d.group_size, N = d.n_sites;
     std::vector<u64> fl(G, 0ULL);
     if (d.flips) std::copy(d.flips, d.flips + G, fl.begin());
-    upload_queued(s.flips, fl);
+    up.add(s.flips, std::move(fl));
     std::vector<double2> ch(G);
     for (int g = 0; g < G; ++g) ch[g] = make_double2(d.chars[2 * g], d.chars[2 * g + 1]);
-    upload_queued(s.chars, ch);
+    up.add(s.chars, std::move(ch));
     s.chars_host.assign(d.chars, d.chars + 2 * G);
     const SlcHost slc = build_slc(d.perms, reinterpret_cast<const u64*>(d.flips), G, N, d.sublattice_mode);
     s.slc_on = slc.on ? 1 : 0;
@@ -599,7 +617,7 @@ void upload_group(qb_sector& s, const qb_sector_desc& d) {
         s.slc_m = slc.m;
         s.slc_contig = slc.contig ? 1 : 0;
         for (int j = 0; j < slc.m; ++j) s.slc_bmask[j] = slc.bmask[j];
-        upload_queued(s.to_key, slc.to_key);
+        up.add(s.to_key, slc.to_key);
         std::vector<u64> pack(slc.lead.size());
         for (std::size_t i = 0; i < pack.size(); ++i) {
             const u64 cnt = slc.cand_off[i + 1] - slc.cand_off[i];
@@ -607,18 +625,18 @@ void upload_group(qb_sector& s, const qb_sector_desc& d) {
             const u64 pay = cnt == 1 ? slc.cand[slc.cand_off[i]] : slc.cand_off[i];
             pack[i] = static_cast<u64>(slc.lead[i]) | (cnt << 16) | (pay << 32);
         }
-        upload_queued(s.lead_pack, pack);
-        upload_queued(s.cand, slc.cand);
+        up.add(s.lead_pack, std::move(pack));
+        up.add(s.cand, slc.cand);
     }
     std::vector<u64> desc, mask;
     s.gkind = classify_group(d.perms, G, N, s.Lx, desc, mask);
     if (s.gkind) {
-        upload_queued(s.edesc, desc);
-        upload_queued(s.emask, mask);
+        up.add(s.edesc, std::move(desc));
+        up.add(s.emask, std::move(mask));
     } else {   // only a group without an arithmetic action reads its byte tables
-        upload_queued(s.lut, build_lut(d.perms, G, N));
+        up.add(s.lut, build_lut(d.perms, G, N));
     }
-    build_pair_table(s, d);
+    build_pair_table(s, d, up);
 }
 
 void validate(const qb_sector_desc* d) {
@@ -647,7 +665,7 @@ void validate(const qb_sector_desc* d) {
 
 // The lookup structure: a rank table indexed by the combinadic rank, or state buckets over the
 // ascending representatives (include/ed/basis/rep_sector.h:85-117, 275-307).
-void build_lookup(qb_sector& s, int want) {
+void build_lookup(qb_sector& s, int want, QueuedUploads& up) {
     if (s.dim == 0) {
         s.lookup = 0;
         return;
@@ -703,7 +721,7 @@ void build_lookup(qb_sector& s, int want) {
         cuda_check(cudaGetLastError(), "hash insert");
     } else if (mode == QB_LOOKUP_RANK) {
         if (s.dim >= (1ULL << 31)) throw Error(QB_EUNSUPPORTED, "rank table: more than 2^31 representatives");
-        upload_queued(s.rank_lut, build_rank_lut(s.N));
+        up.add(s.rank_lut, build_rank_lut(s.N));
         s.rank_table.alloc(static_cast<std::size_t>(ranks));
         cuda_check(cudaMemset(s.rank_table.p, 0xFF, ranks * 4), "rank table clear");
         s.lookup = 1;
@@ -731,7 +749,6 @@ void build_lookup(qb_sector& s, int want) {
                                                                               s.bucket_off.p);
         cuda_check(cudaGetLastError(), "buckets");
     }
-    cuda_check(cudaStreamSynchronize(nullptr), "lookup build");
 }
 
 }  // namespace
@@ -847,11 +864,12 @@ int qb_sector_create(const qb_sector_desc* d, qb_sector** out) {
         s->G = d->group_size;
         s->bpw = (d->n_sites + 7) / 8;
         keep_desc(*s, *d);
-        upload_group(*s, *d);
-        const auto Ch = pascal();
+        QueuedUploads up;
+        upload_group(*s, *d, up);
+        auto Ch = pascal();
         const u64 total = Ch[s->N * 65 + s->n_up];
         DevBuf<u64> C;
-        upload_queued(C, Ch);
+        up.add(C, std::move(Ch));
         // chunks of consecutive ranks, a thread each: at least a thread per resident slot of the chip (2048 an SM)
         // down to 4 states a chunk, up to 64 states a chunk, and beyond that at most 8 chunks a slot. A chunk's states
         // follow one another in one thread, so 64 states a chunk left a 12,870-state scan (chain 16) on 201 threads:
@@ -888,8 +906,8 @@ int qb_sector_create(const qb_sector_desc* d, qb_sector** out) {
                                                    s->inv_norms.p);
             cuda_check(cudaGetLastError(), "enumeration (write)");
         }
-        build_lookup(*s, d->lookup);
-        cuda_check(cudaStreamSynchronize(nullptr), "sector");
+        build_lookup(*s, d->lookup, up);
+        up.finish();
         *out = s.release();
     });
 }
@@ -907,11 +925,13 @@ int qb_sector_create_from_reps(const qb_sector_desc* d, const uint64_t* reps, co
         s->G = d->group_size;
         s->bpw = (d->n_sites + 7) / 8;
         keep_desc(*s, *d);
-        upload_group(*s, *d);
+        QueuedUploads up;
+        upload_group(*s, *d, up);
         s->dim = dim;
         s->reps.upload(reinterpret_cast<const u64*>(reps), dim);
         s->inv_norms.upload(inv_norms, dim);
-        build_lookup(*s, d->lookup);
+        build_lookup(*s, d->lookup, up);
+        up.finish();
         *out = s.release();
     });
 }
