@@ -1201,15 +1201,19 @@ int csr_build(const qb_sector* row, const qb_sector* col, const qb_program* prog
             *out = A.release();
             return;
         }
+        // the sliced copy, whichever way the matrix was built; then the wait: the last copies (device to device: the host
+        // does not wait for them) and the slices are queued on this thread's stream, and the matrix may be read on any
+        // other as soon as the call returns
+        auto done = [&] {
+            if (slices) build_slices(A.get(), max_bytes);
+            cuda_check(cudaStreamSynchronize(nullptr), "CSR build");
+            *out = A.release();
+        };
         const bool narrow = row->N <= 32 && col->N <= 32;
         keep_pool_scratch();
         if (narrow ? build_slabs<u32>(row, col, prog, max_bytes, A.get())
                    : build_slabs<u64>(row, col, prog, max_bytes, A.get())) {
-            if (slices) build_slices(A.get(), max_bytes);
-            // the last copies (device to device: the host does not wait for them) and the slices are queued on this
-            // thread's stream, and the matrix may be read on any other as soon as the call returns
-            cuda_check(cudaStreamSynchronize(nullptr), "CSR build");
-            *out = A.release();
+            done();
             return;
         }
         // flags: [0] a row past 256 entries, [1] dictionary overflow, [2] values inserted, [3] dictionary size
@@ -1283,7 +1287,7 @@ int csr_build(const qb_sector* row, const qb_sector* col, const qb_program* prog
             A->ids.release();
             check_budget(row->dim, A->nnz, 0, 0, max_bytes);
         }
-        *out = A.release();
+        done();
     });
 }
 

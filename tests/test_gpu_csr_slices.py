@@ -1,6 +1,7 @@
 """The sliced one-vector CSR apply of large sectors against the CSR's own kernels on the same entries (an uploaded CSR has no
 sliced copy): FP64 storage bit for bit, FP32 storage within the rounding of its output (1.2e-7). Row counts that are no
-multiple of a slice or a block, rows of 1 to 75 entries, complex values, and a matrix between two sectors."""
+multiple of a slice or a block, rows of 1 to 75 entries, complex values, and a matrix between two sectors; and the same copy
+whichever way the matrix was built."""
 import numpy as np
 import pytest
 
@@ -50,3 +51,33 @@ def test_sliced_apply(name, spec, prog, two):
     A.matvec(x, y, dtype="c64")
     B.matvec(x, z, dtype="c64")
     assert float((y - z).abs().max()) <= 1.2e-7 * float(z.abs().max())
+
+
+def test_slices_of_a_matrix_built_the_general_way():
+    """A budget with room for the merged entries and their slices, not for the entries before the merge (most of them exact
+    zeros: flips that act only with the next two sites up), sends the build the general way. The same apply follows."""
+    from qed_spin_b200 import device as D
+    n = 24
+    prods = []
+    for i in range(n):
+        j, k, m = (i + 1) % n, (i + 2) % n, (i + 3) % n
+        for a, b in ((i, j), (j, i)):   # S+ S- (1/2 + Sz)(1/2 + Sz)
+            prods += [("+-", [a, b], 0.25), ("+-z", [a, b, k], 0.5), ("+-z", [a, b, m], 0.5), ("+-zz", [a, b, k, m], 1.0)]
+    S = D.Sector(lat.chain_sector(n, 12, 5))
+    P = D.Program(ops.row_program(ops.from_products(n, prods)))
+    A = D.Csr(S, S, P)
+    info = A.info()
+    reps = S.reps()[0]
+    flips = sum(int((((reps >> np.uint64(i)) ^ (reps >> np.uint64((i + 1) % n))) & np.uint64(1)).sum()) for i in range(n))
+    unmerged = (S.dim + 1) * 8 + ((flips + 3) & ~3) * 5 + 256 * 16
+    budget = (S.dim + 1) * 8 + (info["nnz"] + 4) * 9 + 256 * 16
+    assert budget < unmerged and info["n_dict"] <= 256
+    B = D.Csr(S, S, P, max_bytes=budget)
+    assert B.info()["bytes"] >= (S.dim + 1) * 8 + info["nnz"] * 9
+    for a, b in zip(A.download(), B.download()):
+        assert np.array_equal(a, b)
+    x = torch.randn(S.dim, dtype=torch.complex64, device="cuda")
+    y, z = torch.empty_like(x), torch.empty_like(x)
+    A.matvec(x, y, dtype="c64")
+    B.matvec(x, z, dtype="c64")
+    assert torch.equal(torch.view_as_real(y).view(torch.int32), torch.view_as_real(z).view(torch.int32))
