@@ -148,3 +148,29 @@ def test_thermal_requests_served():
             r = np.asarray(ref[key])
             np.testing.assert_allclose(g[key], r, rtol=1e-8, atol=1e-8 * max(np.abs(r).max(), 1e-3), err_msg=key)
     assert got[3]["converged"] and len(got[3]["values"]) == 2
+
+
+def test_footprint_holds_the_csr_builds_scratch():
+    """A request on a sector the one-walk CSR build takes (112,720 rows) is admitted with room for that build's slab (21 bytes
+    a row and group), and its levels equal a direct call's; two of them do not run together under a budget of one and
+    a half footprints."""
+    from qed_spin_b200 import device as D
+    n = 24
+    h = ops.row_program(ops.from_products(n, ops.heisenberg_products(lat.chain_bonds(n))))
+    spec = lat.chain_sector(n, 12, 0)
+    S, P = D.Sector(spec), D.Program(h)
+    A = D.Csr(S, S, P)
+    A.attach(P)
+    srv = D.Server(max_active=1)
+    one = srv.wait(srv.submit_eigs(spec, h, 1))
+    srv.close()
+    vectors = 48 * S.dim
+    assert one["footprint"] >= A.info()["nnz"] * 5 + S.dim * 21 * h.n_groups > vectors + A.info()["nnz"] * 5
+    assert np.array_equal(_bits(one["values"]), _bits([D.eigs_lowest(S, P)["e0"]]))
+    srv = D.Server(max_active=4, hbm_budget=int(1.5 * one["footprint"]))
+    got = [srv.wait(t) for t in [srv.submit_eigs(spec, h, 1) for _ in range(3)]]
+    srv.close()
+    for g in got:
+        assert np.array_equal(_bits(g["values"]), _bits(one["values"]))
+    spans = sorted((g["t_admit"], g["t_done"]) for g in got)
+    assert all(a[1] <= b[0] for a, b in zip(spans, spans[1:]))
