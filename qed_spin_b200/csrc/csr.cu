@@ -1048,8 +1048,9 @@ void build_slices(qb_csr* A, uint64_t max_bytes) {
     cuda_check(cudaGetLastError(), "CSR slices");
 }
 
-// ... and at most this much scratch, an eighth of the free memory at most.
+// ... and at most this much scratch, an eighth of the free memory at most, and what a server's worker was admitted with.
 constexpr std::size_t kSlabBytes = std::size_t{2} << 30;
+std::size_t slab_row_bytes(u64 groups) { return static_cast<std::size_t>(groups) * (4 + 16 + 1) + 4 + 8; }
 
 void slab_merge(int held, unsigned blocks, std::size_t smem, u64 n, const SlabEntries& E, unsigned long long* counts,
                 const SlabSet& D) {
@@ -1096,13 +1097,13 @@ bool build_slabs(const qb_sector* row, const qb_sector* col, const qb_program* P
         u64 most = 0;
         cuda_check(cudaMemcpy(&most, total.p, 8, cudaMemcpyDeviceToHost), "CSR bound");
         // chunks of equal length
-        const std::size_t per_row = static_cast<std::size_t>(cap) * (4 + 16 + 1) + 4 + 8;
+        const std::size_t per_row = slab_row_bytes(cap);
         const std::size_t need = (dim + 1) * 8 + padded(most) * 5 + 256 * 16;
         if (max_bytes && need > max_bytes) return false;
         std::size_t free_b = 0, total_b = 0;
         cuda_check(cudaMemGetInfo(&free_b, &total_b), "cudaMemGetInfo");
         if (need > free_b + idle_cached_bytes()) return false;
-        const u64 fit = std::min(kSlabBytes, free_b / 8) / per_row;
+        const u64 fit = std::min({kSlabBytes, free_b / 8, scratch_limit()}) / per_row;
         if (fit < kSlabMinRows / 2) return false;
         const u64 n_chunks = (dim + fit - 1) / fit;
         const u64 chunk = (dim + n_chunks - 1) / n_chunks;
@@ -1150,6 +1151,9 @@ bool build_slabs(const qb_sector* row, const qb_sector* col, const qb_program* P
             cuda_check(cudaMemcpy(A->vals.p, dict.p, n_dict * 16, cudaMemcpyDeviceToDevice), "dictionary copy");
             A->n_dict = static_cast<int>(n_dict);
             A->id_bytes = 1;
+            scol.release();
+            sval.release();
+            sid.release();
             if (padded(A->nnz) + A->nnz / 16 < A->col_idx.n) {   // many merged entries: arrays of their own length
                 DevBuf<u32> c(padded(A->nnz));
                 DevBuf<unsigned char> i(padded(A->nnz));
@@ -1172,6 +1176,11 @@ bool build_slabs(const qb_sector* row, const qb_sector* col, const qb_program* P
 }
 
 }  // namespace
+
+std::uint64_t csr_build_scratch(std::uint64_t rows, std::uint32_t groups) {
+    if (rows < kSlabMinRows || groups < 1 || groups > static_cast<std::uint32_t>(kMaxRowEntries)) return 0;
+    return std::min<std::uint64_t>(kSlabBytes, rows * slab_row_bytes(groups));
+}
 
 void csr_spmv(const qb_csr* A, const void* in, void* out, int k, int dtype_in, int dtype_out, cudaStream_t st) {
     if (A->rows == 0) return;

@@ -48,7 +48,10 @@ void set_last_error(const std::string& m);
 // the free device memory, or less when the thread has an allowance (a request server's worker sets one to
 // the footprint it admitted the request with; 0: none).
 std::size_t available_bytes();
-void set_thread_allowance(std::size_t bytes);
+// scratch: the most a CSR build of this thread may take beside the matrix (a worker sets what it admitted the request
+// with; 0: none set, scratch_limit() is the free device memory).
+void set_thread_allowance(std::size_t bytes, std::size_t scratch = 0);
+std::size_t scratch_limit();
 
 // The launch shape of a kernel family for a size-class key (tune.cu): a forced or known choice, or -- when
 // measuring and st is not capturing -- the fastest of n candidates, each run by run(c) on st; else fallback.
@@ -278,6 +281,9 @@ void csr_spmv(const qb_csr* A, const void* in, void* out, int k, int dtype_in, i
 // qb_csr_build; slices: with the sliced copy that one-vector applies read (the batched recurrences read the CSR itself).
 int csr_build(const qb_sector* row, const qb_sector* col, const qb_program* prog, std::uint64_t max_bytes, bool slices,
               qb_csr** out);
+// The scratch that csr_build takes for a sector of `rows` rows and a program of `groups` groups when it is free to (0: it
+// takes the general path).
+std::uint64_t csr_build_scratch(std::uint64_t rows, std::uint32_t groups);
 }  // namespace qb
 
 namespace qb {

@@ -26,8 +26,13 @@ namespace qb {
 thread_local std::string g_last_error;
 void set_last_error(const std::string& m) { g_last_error = m; }
 
-thread_local std::size_t g_allowance = 0;
-void set_thread_allowance(std::size_t bytes) { g_allowance = bytes; }
+thread_local std::size_t g_allowance = 0, g_scratch = 0;
+void set_thread_allowance(std::size_t bytes, std::size_t scratch) { g_allowance = bytes, g_scratch = scratch; }
+std::size_t scratch_limit() {
+    std::size_t free_b = 0, total_b = 0;
+    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) free_b = 0;
+    return g_allowance ? std::min(free_b, g_scratch) : free_b;
+}
 std::size_t available_bytes() {
     std::size_t free_b = 0, total_b = 0;
     if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) free_b = 0;

@@ -84,7 +84,7 @@ struct Job {
     double eta = 0.05;
     int samples = 0;
     std::uint64_t seed = 0;
-    std::uint64_t footprint = 0, allowance = 0, csr_budget = 0;
+    std::uint64_t footprint = 0, allowance = 0, csr_budget = 0, scratch = 0;
     double t_submit = 0.0, t_admit = -1.0, t_done = -1.0;
     bool done = false;
     int status = QB_OK;
@@ -132,8 +132,13 @@ void plan(Job& j, std::uint64_t budget) {
         work = 96 * n + 64 * nt;   // ground state: seed, w, u and the recurrence; phi and the fraction's recurrence
         keep = std::min<std::uint64_t>(610 * 16 * n, budget / 8);   // a kept basis for the ground state's Ritz vector
     }
+    // A CSR's build takes its scratch, and then for a moment a second copy of the matrix (the trim of merged entries), before
+    // the solve's vectors are there.
+    const std::uint64_t rows = j.kind == QB_REQ_DYNAMICS ? std::max(n, estimate_dim(j.tgt.d)) : n;
+    j.scratch = csr_build_scratch(rows, j.h.d.n_groups);
+    const std::uint64_t build = j.scratch ? std::max(j.scratch, csr_bytes(rows, j.h.d)) : 0;
     j.csr_budget = csr;
-    j.footprint = fixed + csr + work + keep;
+    j.footprint = fixed + csr + std::max(work + keep, build);
     // what the solve may plan its optional buffers with: the kept basis it was admitted with, as the lanes'
     // half-of-available rule reads it
     j.allowance = 2 * (keep + work) + 1;
@@ -180,7 +185,7 @@ struct qb_server {
                 ++active;
                 j->t_admit = now();
             }
-            qb::set_thread_allowance(j->allowance);
+            qb::set_thread_allowance(j->allowance, j->scratch);
             run(*j);
             qb::set_thread_allowance(0);
             {

@@ -14,6 +14,8 @@
 // =============================================================================
 #include <algorithm>
 #include <cstdint>
+#include <random>
+#include <vector>
 
 #include "qb_internal.cuh"
 
@@ -167,6 +169,10 @@ __global__ void __launch_bounds__(kPolarThreads) k_polar_write(const ulonglong2*
     }
 }
 
+// Up to this many entries the host draws them: the device's four launches and its wait take about 60 us whatever the number,
+// the host 0.06 us an entry (the lowest level of 8 states: 1.08 ms with the host's draw, 1.13 with the device's).
+constexpr std::uint64_t kHostEntries = 512;
+
 // A pass of the draw: at most 1 M attempts, 16 MB of raw outputs.
 constexpr u64 kPassBlocks = (u64{1} << 20) / (kN / 2);
 
@@ -175,6 +181,17 @@ constexpr u64 kPassBlocks = (u64{1} << 20) / (kN / 2);
 // out[0, n): the staged start of the seed, queued on st; returns when it is complete.
 void staged_start_device(double2* out, std::uint64_t n, std::uint64_t seed, cudaStream_t st) {
     if (n == 0) return;
+    if (n <= kHostEntries) {
+        std::vector<double2> v(n);
+        std::mt19937_64 gen(seed);
+        std::normal_distribution<double> normal(0.0, 1.0);
+        for (double2& z : v) {
+            z.y = normal(gen);   // the imaginary part is drawn first
+            z.x = normal(gen);
+        }
+        upload_host(out, v.data(), n * 16, st);
+        return;
+    }
     // pi/4 of the attempts are accepted: the expected number and a margin, in whole generator blocks of 156 attempts
     auto blocks_for = [](u64 left) {
         const u64 a = left + left / 4 + left / 32 + 1024;
