@@ -754,8 +754,8 @@ __global__ void __launch_bounds__(256) k_slice(u64 rows, const unsigned long lon
     }
 }
 
-template <bool kInF32, bool kOutF32>
-__global__ void __launch_bounds__(256) spmv1_sliced(u64 rows, const unsigned long long* __restrict__ row_ptr,
+template <bool kInF32, bool kOutF32, bool kTight>
+__global__ void __launch_bounds__(256, kTight ? 6 : 0) spmv1_sliced(u64 rows, const unsigned long long* __restrict__ row_ptr,
                                                     const u32* __restrict__ slices, int bits,
                                                     const double2* __restrict__ vals, int n_dict, const void* in_v,
                                                     void* out_v) {
@@ -773,7 +773,7 @@ __global__ void __launch_bounds__(256) spmv1_sliced(u64 rows, const unsigned lon
     const u32 cmask = (1u << bits) - 1u;
     u64 base = __shfl_sync(0xffffffffu, f0, 0);
     const int most = __reduce_max_sync(0xffffffffu, len);
-    constexpr int U = kInF32 ? 4 : 2;   // entries in flight a row (a sweep of 2, 4, 6 and 8)
+    constexpr int U = !kInF32 ? 2 : kTight ? 3 : 4;   // entries in flight a row (a sweep of 2, 4, 6 and 8)
     u32 e[U];
     auto fetch = [&](int q0) {   // the words of entries q0 .. q0 + U - 1
 #pragma unroll
@@ -915,13 +915,44 @@ bool team32_for(const qb_csr* A) {
     return A->rows > 0 && A->nnz >= kTeamMinRow * A->rows;
 }
 
+// The rows that the kernel's resident blocks hold at once, a thread a row.
+template <class K> u64 rows_at_once(K kernel) {
+    int dev = 0, sms = 148, per_sm = 0;
+    cuda_check(cudaGetDevice(&dev), "device");
+    cuda_check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "SM count");
+    cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 256, 0), "occupancy");
+    return static_cast<u64>(sms) * per_sm * 256;
+}
+
+// The form of the sliced apply: 1 the usual one, 2 the tight one (six blocks an SM), 0 the CSR's own kernels. A row's loads
+// are a chain that a last wave of a few blocks runs through as slowly as a full one, so FP32 storage, whose usual form has
+// five blocks an SM (189 k rows at once), takes the tight form where that makes one wave of two (208 k rows of 53
+// entries: 42.4 -> 32.6 us, of 27 entries 22.6 -> 18.5; everywhere else it is up to 7% slower), and behind it, up to a
+// quarter of a second wave, four lanes a row where those serve (6x6 at 7 spins up, 232 k rows: 38.1 -> 35.7 us).
+template <bool kInF32, bool kOutF32> int sliced_form(const qb_csr* A) {
+    if (!A->slices.n || team_force() >= 0) return 0;
+    if constexpr (kInF32) {
+        static const u64 usual = rows_at_once(spmv1_sliced<kInF32, kOutF32, false>),
+                         tight = rows_at_once(spmv1_sliced<kInF32, kOutF32, true>);
+        if (A->rows > usual && A->rows <= tight) return 2;
+        if (A->rows > usual && A->rows <= usual + usual / 4 && team32_for(A)) return 0;
+    }
+    return 1;
+}
+
 template <bool kInF32, bool kOutF32>
 void spmv_launch(const qb_csr* A, const void* in, void* out, int k, cudaStream_t st) {
     const unsigned char* ids = A->ids.p;
     const double2* vals = A->vals.p;
-    if (k == 1 && A->slices.n && team_force() < 0) {
-        spmv1_sliced<kInF32, kOutF32><<<static_cast<unsigned>((A->rows + 255) / 256), 256, 0, st>>>(
-            A->rows, A->row_ptr.p, A->slices.p, A->slice_bits, vals, A->n_dict, in, out);
+    const int sliced = k == 1 ? sliced_form<kInF32, kOutF32>(A) : 0;
+    if (sliced) {
+        auto go = [&](auto kernel) {
+            kernel<<<static_cast<unsigned>((A->rows + 255) / 256), 256, 0, st>>>(A->rows, A->row_ptr.p, A->slices.p,
+                                                                               A->slice_bits, vals, A->n_dict, in, out);
+        };
+        if constexpr (kInF32)
+            if (sliced == 2) go(spmv1_sliced<kInF32, kOutF32, true>);
+        if (sliced == 1) go(spmv1_sliced<kInF32, kOutF32, false>);
     } else if (k == 1 && kInF32 && A->id_bytes == 1 && team32_for(A)) {
         const u64 threads = A->rows * kTeamLanes;
         spmv1_team32<kOutF32><<<static_cast<unsigned>((threads + 255) / 256), 256, 0, st>>>(

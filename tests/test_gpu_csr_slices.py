@@ -1,7 +1,7 @@
 """The sliced one-vector CSR apply of large sectors against the CSR's own kernels on the same entries (an uploaded CSR has no
 sliced copy): FP64 storage bit for bit, FP32 storage within the rounding of its output (1.2e-7). Row counts that are no
-multiple of a slice or a block, rows of 1 to 75 entries, complex values, and a matrix between two sectors; and the same copy
-whichever way the matrix was built."""
+multiple of a slice or a block, rows of 1 to 75 entries, complex values, a matrix between two sectors, and row counts on
+both sides of each form's last wave; and the same copy whichever way the matrix was built."""
 import numpy as np
 import pytest
 
@@ -20,16 +20,19 @@ def _chain(n, jz=0.7, chiral=0.0):
     return ops.row_program(ops.from_products(n, prods))
 
 
-def _square():
-    nn, nnn = lat.square_j1j2_bonds(6, 4)
-    return ops.row_program(ops.from_products(24, ops.heisenberg_products(nn) + ops.heisenberg_products(nnn, 0.5)))
+def _square(Lx=6, Ly=4):
+    nn, nnn = lat.square_j1j2_bonds(Lx, Ly)
+    return ops.row_program(ops.from_products(Lx * Ly, ops.heisenberg_products(nn) + ops.heisenberg_products(nnn, 0.5)))
 
 
 @pytest.mark.parametrize("name,spec,prog,two", [
     ("chiral", lat.chain_sector(24, 11, 5), lambda: _chain(24, chiral=0.2), False),
     ("no diagonal", lat.chain_sector(25, 9, 0), lambda: _chain(25, jz=0.0), False),
     ("square", lat.square_k0_sector(6, 4, 12), _square, False),
-    ("two handles", lat.chain_sector(24, 12, 3), lambda: _chain(24), True)], ids=lambda v: v if isinstance(v, str) else "")
+    ("two handles", lat.chain_sector(24, 12, 3), lambda: _chain(24), True),
+    ("six blocks an SM", lat.chain_sector(26, 10, 1), lambda: _chain(26), False),          # 204 k rows on 148 SMs
+    ("a short second wave", lat.square_k0_sector(6, 6, 7), lambda: _square(6, 6), False),   # 232 k rows of 47 entries
+    ("a second wave", lat.chain_sector(28, 9, 3), lambda: _chain(28, chiral=0.2), False)], ids=lambda v: v if isinstance(v, str) else "")
 def test_sliced_apply(name, spec, prog, two):
     if not torch.cuda.is_available():
         pytest.fail("a GPU test ran without a CUDA device")
