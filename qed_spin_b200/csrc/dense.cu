@@ -32,6 +32,10 @@ namespace {
 constexpr int kDenseDeviceMax = 1024;   // four vectors of 16-byte elements in shared memory, a row a thread
 constexpr int kDenseThreads = 1024;
 static_assert(kDenseThreads >= kDenseDeviceMax, "a thread holds at most one row of a column");
+// Launches whose largest block has at most this many states: 256 threads, whose barriers and sums of the warps' sums are
+// shorter (one block, us, 1,024 against 256 threads: 12 states 188 / 165, 28 338 / 279, 56 828 / 727; 126 states 1,548 / 1,421,
+// 210 3,478 / 3,489).
+constexpr int kDenseFew = 64, kDenseFewThreads = 256;
 
 struct DenseBlock {
     unsigned long long a_off;   // the block's matrix at A + a_off (column-major, n x n)
@@ -121,7 +125,8 @@ __device__ int sturm_below(const double* d, const double* e, int n, double x) {
 // elements in flight. The 238 dense blocks of a 16-site chain (64 of about 500 states, side by side): 23 ms, where two
 // passes over A22 a step (p, then the update), 256 threads and a thread per row of p took 145 ms.
 constexpr std::size_t kDenseSmem = (4 * static_cast<std::size_t>(kDenseDeviceMax) * 16) + 64 * 8;
-__global__ void __launch_bounds__(kDenseThreads, 1) k_dense_levels(const DenseBlock* blocks, double2* A_all,
+template <int kThreads>
+__global__ void __launch_bounds__(kThreads, 1) k_dense_levels(const DenseBlock* blocks, double2* A_all,
                                                                    double* values) {
     extern __shared__ __align__(16) unsigned char smem[];
     double2* v = reinterpret_cast<double2*>(smem);       // the pending update A22 -= 2 (v w^H + w v^H)
@@ -133,7 +138,7 @@ __global__ void __launch_bounds__(kDenseThreads, 1) k_dense_levels(const DenseBl
     __shared__ double s_lo, s_hi;
     const DenseBlock B = blocks[blockIdx.x];
     const int n = B.n, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    constexpr int kWarps = kDenseThreads / 32;
+    constexpr int kWarps = kThreads / 32;
     double2* A = A_all + B.a_off;
     auto col = [&](int c) { return A + static_cast<std::size_t>(c) * n; };
     // a - 2 (vi conj(wj) + wi conj(vj))
@@ -142,10 +147,10 @@ __global__ void __launch_bounds__(kDenseThreads, 1) k_dense_levels(const DenseBl
         a.y -= 2.0 * ((vi.y * wj.x - vi.x * wj.y) + (wi.y * vj.x - wi.x * vj.y));
         return a;
     };
-    for (int i = threadIdx.x; i < n; i += kDenseThreads) v[i] = w[i] = make_double2(0.0, 0.0);
+    for (int i = threadIdx.x; i < n; i += kThreads) v[i] = w[i] = make_double2(0.0, 0.0);
     __syncthreads();
     for (int k = 0; k < n; ++k) {
-        // column k with the pending update; a thread keeps its rows' elements (n <= kDenseDeviceMax = the threads)
+        // column k with the pending update; a thread keeps its row's element (n is at most the threads)
         const int i0 = k + threadIdx.x;
         double2 x = make_double2(0.0, 0.0);
         if (i0 < n) x = updated(col(k)[i0], v[i0], w[i0], v[k], w[k]);
@@ -254,7 +259,7 @@ __global__ void __launch_bounds__(kDenseThreads, 1) k_dense_levels(const DenseBl
         s_hi = hi + pad;
     }
     __syncthreads();
-    for (int q = threadIdx.x; q < n; q += kDenseThreads) {
+    for (int q = threadIdx.x; q < n; q += kThreads) {
         double lo = s_lo, hi = s_hi;
         for (int it = 0; it < 200; ++it) {
             const double mid = 0.5 * (lo + hi);
@@ -271,7 +276,8 @@ __global__ void __launch_bounds__(kDenseThreads, 1) k_dense_levels(const DenseBl
 // Launches k_assemble over the blocks of `set`.
 template <class ST>
 void assemble(const std::vector<int>& set, const qb_sector* const* secs, const qb_program* const* progs,
-              const std::vector<std::uint64_t>& a_off, double2* A, DevBuf<AsmItem>& d_items, DevBuf<AsmTile>& d_tiles) {
+              const std::vector<std::uint64_t>& a_off, double2* A, DevBuf<AsmItem>& d_items, DevBuf<AsmTile>& d_tiles,
+              QueuedUploads& up) {
     if (set.empty()) return;
     std::vector<AsmItem> items;
     std::vector<AsmTile> tiles;
@@ -283,10 +289,11 @@ void assemble(const std::vector<int>& set, const qb_sector* const* secs, const q
             tiles.push_back(AsmTile{static_cast<int>(items.size()), static_cast<u32>(r)});
         items.push_back(AsmItem{secs[b]->view(), progs[b]->view, a_off[b], in_smem ? 1 : 0});
     }
-    d_items.upload(items);
-    d_tiles.upload(tiles);
+    const unsigned n_tiles = static_cast<unsigned>(tiles.size());
+    up.add(d_items, std::move(items));
+    up.add(d_tiles, std::move(tiles));
     set_smem(k_assemble<ST>, smem);
-    k_assemble<ST><<<static_cast<unsigned>(tiles.size()), kAsmRows, smem, cudaStreamPerThread>>>(d_items.p, d_tiles.p, A);
+    k_assemble<ST><<<n_tiles, kAsmRows, smem, cudaStreamPerThread>>>(d_items.p, d_tiles.p, A);
     cuda_check(cudaGetLastError(), "dense assembly");
 }
 
@@ -315,8 +322,9 @@ bool dense_levels_device(const qb_sector* const* secs, const qb_program* const* 
     cuda_check(cudaMemsetAsync(A.p, 0, a_tot * 16, cudaStreamPerThread), "dense clear");
     DevBuf<AsmItem> d_items[2];
     DevBuf<AsmTile> d_tiles[2];
-    assemble<u32>(walk_set[0], secs, progs, a_off, A.p, d_items[0], d_tiles[0]);
-    assemble<u64>(walk_set[1], secs, progs, a_off, A.p, d_items[1], d_tiles[1]);
+    QueuedUploads up;
+    assemble<u32>(walk_set[0], secs, progs, a_off, A.p, d_items[0], d_tiles[0], up);
+    assemble<u64>(walk_set[1], secs, progs, a_off, A.p, d_items[1], d_tiles[1], up);
     for (int b = 0; b < n_blocks; ++b)
         if (const qb_csr* C = secs[b]->dim ? csr_lane(secs[b], secs[b], progs[b]) : nullptr)
             k_assemble_csr<<<static_cast<unsigned>((C->rows + 127) / 128), 128, 0, cudaStreamPerThread>>>(
@@ -328,14 +336,22 @@ bool dense_levels_device(const qb_sector* const* secs, const qb_program* const* 
     std::vector<DenseBlock> sorted(desc.size());
     for (std::size_t i = 0; i < order.size(); ++i) sorted[i] = desc[order[i]];
     DevBuf<DenseBlock> dd;
-    dd.upload(sorted.data(), sorted.size());
+    const unsigned n_desc = static_cast<unsigned>(sorted.size());
+    const int most = sorted.front().n;
+    up.add(dd, std::move(sorted));
     DevBuf<double> dv(v_tot);
-    set_smem(k_dense_levels, kDenseSmem);
-    k_dense_levels<<<static_cast<unsigned>(sorted.size()), kDenseThreads, kDenseSmem, cudaStreamPerThread>>>(dd.p, A.p,
-                                                                                                           dv.p);
+    auto go = [&](auto kernel, int threads) {
+        set_smem(kernel, kDenseSmem);
+        kernel<<<n_desc, threads, kDenseSmem, cudaStreamPerThread>>>(dd.p, A.p, dv.p);
+    };
+    if (most <= kDenseFew)
+        go(k_dense_levels<kDenseFewThreads>, kDenseFewThreads);
+    else
+        go(k_dense_levels<kDenseThreads>, kDenseThreads);
     cuda_check(cudaGetLastError(), "dense levels");
     std::vector<double> hv(v_tot);
     cuda_check(cudaMemcpy(hv.data(), dv.p, v_tot * 8, cudaMemcpyDeviceToHost), "dense levels");
+    up.finish();
     for (const auto& d : desc) std::copy(hv.begin() + d.v_off, hv.begin() + d.v_off + d.n, values + d.v_off);
     return true;
 }

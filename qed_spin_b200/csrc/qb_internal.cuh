@@ -22,6 +22,7 @@
 #include <atomic>
 #include <cstdint>
 #include <functional>
+#include <memory>
 #include <stdexcept>
 #include <string>
 #include <vector>
@@ -128,6 +129,31 @@ template <class T> struct DevBuf {
     }
     void upload(const std::vector<T>& v) { upload(v.data(), v.size()); }
     std::size_t bytes() const { return n * sizeof(T); }
+};
+
+// Small host tables copied to the device in the order of the calling thread's stream: each is kept here until finish() has
+// waited for the copies, since nothing promises that a pageable source has been read when the call that queues its copy
+// returns. One wait for them all: with a synchronisation each, a dozen tables were a third of a small sector's creation.
+class QueuedUploads {
+public:
+    ~QueuedUploads() {
+        if (!held_.empty()) cudaStreamSynchronize(cudaStreamPerThread);   // left by an exception
+    }
+    template <class T> void add(DevBuf<T>& b, std::vector<T> v) {
+        b.alloc(v.size());
+        if (v.empty()) return;
+        const auto keep = std::make_shared<std::vector<T>>(std::move(v));
+        held_.push_back(keep);
+        cuda_check(cudaMemcpyAsync(b.p, keep->data(), keep->size() * sizeof(T), cudaMemcpyHostToDevice, cudaStreamPerThread),
+                   "upload");
+    }
+    void finish() {
+        cuda_check(cudaStreamSynchronize(cudaStreamPerThread), "uploads");
+        held_.clear();
+    }
+
+private:
+    std::vector<std::shared_ptr<void>> held_;
 };
 
 // ---------------------------------------------------------------------------------------------

@@ -15,7 +15,6 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
-#include <memory>
 #include <mutex>
 #include <numeric>
 
@@ -554,31 +553,6 @@ int classify_group(const int32_t* perms, int G, int N, int& Lx, std::vector<u64>
     mask.assign(G, 0ULL);
     return 0;
 }
-
-// The tables of a sector in the making, copied in stream order: each is kept here until finish() has waited for the copies,
-// since nothing promises that a pageable source has been read when the call that queues its copy returns. One wait for
-// them all: with a synchronisation each, a dozen tables were a third of a small sector's creation.
-class QueuedUploads {
-public:
-    ~QueuedUploads() {
-        if (!held_.empty()) cudaStreamSynchronize(cudaStreamPerThread);   // left by an exception
-    }
-    template <class T> void add(DevBuf<T>& b, std::vector<T> v) {
-        b.alloc(v.size());
-        if (v.empty()) return;
-        const auto keep = std::make_shared<std::vector<T>>(std::move(v));
-        held_.push_back(keep);
-        cuda_check(cudaMemcpyAsync(b.p, keep->data(), keep->size() * sizeof(T), cudaMemcpyHostToDevice, cudaStreamPerThread),
-                   "upload");
-    }
-    void finish() {
-        cuda_check(cudaStreamSynchronize(cudaStreamPerThread), "sector");
-        held_.clear();
-    }
-
-private:
-    std::vector<std::shared_ptr<void>> held_;
-};
 
 // The row-pair table (for_each_row_candidate) when the group is every translation of a torus, numbered a + Lx b and
 // without flips, and the key order's blocks are its rows, of at most 6 sites (16 KB), with more than 32 sites (the

@@ -1,6 +1,7 @@
 """The dense tail's one-pass reduction against numpy's dense solve of the oracle's matrix, 1e-11 of the scale: one and two
-states, sizes around a warp and a pair of columns, the largest block the device takes (1,024 states and just below),
-a diagonal operator (zero columns: no reflections), 64-bit states, an attached CSR, and blocks of several programs."""
+states, sizes around a warp, around the largest block of 256 threads (64 states), 1,001 states, exactly the largest block
+the device takes (1,024) and one that the host takes (1,035), a diagonal operator (zero columns: no reflections),
+64-bit states, an attached CSR, and blocks of several programs."""
 import numpy as np
 import pytest
 
@@ -31,9 +32,29 @@ def _chiral(n):
         [(i, (i + 1) % n, (i + 2) % n) for i in range(n)], 0.3)))
 
 
+def _pairs(m):
+    """m disjoint pairs of sites with one spin up in each: 2^m states of 2m sites, closed under flips within a pair."""
+    n = 2 * m
+    prods = []
+    for i in range(m):
+        prods += ops.xxz_products([(2 * i, 2 * i + 1)], 0.4 + 0.1 * i, 0.0)
+        prods += ops.xxz_products([(2 * i, (2 * i + 2) % n)], 0.0, 0.7 + 0.03 * i)
+    reps = np.sort(np.array([sum(1 << (2 * i + ((s >> i) & 1)) for i in range(m)) for s in range(1 << m)], np.uint64))
+    A = np.zeros((len(reps), len(reps)))
+    index = {int(r): i for i, r in enumerate(reps)}
+    for r, i in index.items():
+        up = [((r >> (2 * q)) & 1) - 0.5 for q in range(m)]
+        A[i, i] = sum((0.7 + 0.03 * q) * up[q] * up[(q + 1) % m] for q in range(m))
+        for q in range(m):
+            A[index[r ^ (3 << (2 * q))], i] += 0.5 * (0.4 + 0.1 * q)
+    return _no_symmetry(n, m), ops.row_program(ops.from_products(n, prods)), reps, A
+
+
 CASES = [("one", lat.chain_sector(6, 0, 0), _chiral(6)), ("two", lat.chain_sector(6, 2, 1), _chiral(6)),
          ("k=5", lat.chain_sector(11, 5, 5), _chiral(11)), ("36", _no_symmetry(9, 2), _chiral(9)),
          ("1001", _no_symmetry(14, 4), _chiral(14)), ("35 sites", _no_symmetry(35, 1), _chiral(35)),
+         *((str(n), _no_symmetry(n, 1), _chiral(n)) for n in (31, 32, 33, 63, 64)),
+         ("66", _no_symmetry(12, 2), _chiral(12)), ("1035", _no_symmetry(46, 2), _chiral(46)),
          ("ising", lat.chain_sector(12, 6, 0),
           ops.row_program(ops.from_products(12, ops.xxz_products(lat.chain_bonds(12), 0.0, 1.0))))]
 
@@ -61,3 +82,12 @@ def test_dense_blocks_of_several_sizes_and_state_widths():
         out = D.dense_levels_blocks(secs, D.Program(prog))
         assert np.array_equal(out[0], out[2])
         np.testing.assert_array_equal(out[0], D.dense_levels(secs[0], D.Program(prog)))
+
+
+@pytest.mark.parametrize("m", [6, 10])   # 64 and 1,024 states
+def test_dense_levels_of_exactly_the_limits(m):
+    from qed_spin_b200 import device as D
+    spec, prog, reps, A = _pairs(m)
+    S = D.Sector(spec, reps=reps, inv_norms=np.ones(len(reps)))
+    ref = np.linalg.eigvalsh(A)
+    np.testing.assert_allclose(D.dense_levels(S, D.Program(prog)), ref, rtol=0, atol=1e-11 * np.abs(ref).max())
