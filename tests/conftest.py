@@ -1,6 +1,7 @@
 """Shared test set-up: the `gpu` marker, the golden fixtures, and the checkers under oracle/."""
 import json
 import os
+import subprocess
 import sys
 
 import numpy as np
@@ -25,6 +26,18 @@ def fixtures():
 def golden():
     with open(os.path.join(GOLDEN, "golden.json")) as fh:
         return json.load(fh)
+
+
+def need_reference(lib="libqed_ref.so"):
+    """Goes on when oracle/_ref/`lib` is there: the reference's own code, compiled from its sources (oracle/Makefile, run by
+    __graft_entry__.build()). Skips where neither it nor the sources are, as nothing can be compared there; sources without
+    the library fail."""
+    if os.path.exists(os.path.join(ROOT, "oracle", "_ref", lib)):
+        return
+    r = subprocess.run(["make", "-s", "-C", os.path.join(ROOT, "oracle"), "print-ref"], capture_output=True, text=True)
+    if r.returncode == 0 and os.path.isdir(os.path.join(r.stdout.strip(), "include", "ed")):
+        pytest.fail(f"oracle/_ref/{lib} is not built (oracle/Makefile, run by __graft_entry__.build())")
+    pytest.skip(f"oracle/_ref/{lib} is not here, nor are the reference's sources")
 
 
 def host_program(fx, name):

@@ -5,15 +5,11 @@ import os
 import subprocess
 import sys
 
-import pytest
-
-from conftest import ROOT
+from conftest import ROOT, need_reference
 
 
 def test_reference_arm_line():
-    lib = os.path.join(ROOT, "oracle", "_ref", "libqed_ref.so")
-    if not os.path.exists(lib):
-        pytest.fail("the reference engine library is not built (oracle/Makefile, run by __graft_entry__.build())")
+    need_reference()
     out = subprocess.run([sys.executable, os.path.join(ROOT, "bench.py"), "--impl", "reference", "--steps", "1",
                           "--warmup", "3"], cwd=ROOT, capture_output=True, text=True, timeout=600)
     assert out.returncode == 0, out.stderr[-2000:]

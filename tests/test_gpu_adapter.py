@@ -15,7 +15,7 @@ import numpy as np
 import pytest
 
 from cases import CASES, NAMES
-from conftest import ROOT
+from conftest import ROOT, need_reference
 from qed_spin_b200 import operators as ops
 
 pytestmark = pytest.mark.gpu
@@ -29,8 +29,7 @@ CASE = {c[0]: c for c in CASES}
 def adapter():
     if not torch.cuda.is_available():
         pytest.fail("a GPU test ran without a CUDA device")
-    if not os.path.exists(LIB):
-        pytest.fail("oracle/_ref/libqed_adapter.so is not built (oracle/Makefile, run by __graft_entry__.build())")
+    need_reference("libqed_adapter.so")
     from qed_spin_b200 import build
     build.build()
     L = C.CDLL(LIB)

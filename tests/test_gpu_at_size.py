@@ -19,10 +19,12 @@ compiled from the reference sources) on the very sectors bench.py measures, thro
   ground state (depth 10, 1e-6 of max S).
 """
 import math
+import os
 
 import numpy as np
 import pytest
 
+from conftest import need_reference
 from oracle import oracle as O
 from oracle import ref as R
 from qed_spin_b200 import lattice as lat
@@ -37,11 +39,13 @@ torch = pytest.importorskip("torch")
 def _cuda():
     if not torch.cuda.is_available():
         pytest.fail("a GPU test ran without a CUDA device")
-    if not R.available():
-        pytest.fail("the reference engine's CPU library (oracle/_ref) is not built")
     from qed_spin_b200 import build
     build.build()
-    import os
+
+
+@pytest.fixture()
+def reference():
+    need_reference()
     R.set_threads(os.cpu_count() or 1)
 
 
@@ -58,7 +62,7 @@ def _x(n, seed):
     return rng.normal(size=n) + 1j * rng.normal(size=n)
 
 
-def test_chain32_a1_flip_bit_exact():
+def test_chain32_a1_flip_bit_exact(reference):
     from qed_spin_b200 import device as D
     N = 32
     spec = lat.chain_a1_flip_sector(N)
@@ -96,7 +100,7 @@ def test_chain32_a1_flip_bit_exact():
     assert np.array_equal(_bits(D.matvec_host(S, S, P, x)), _bits(yd.cpu().numpy()))
 
 
-def test_chain32_k2_levels_against_reference():
+def test_chain32_k2_levels_against_reference(reference):
     """The two lowest levels of the chain-32 sector: the k > 1 lane on the device CSR in FP64 storage, and in FP32
     storage with the FP64 refinement, against the reference engine's own krylov_schur_kernel on its host CSR
     (1e-9 of the coupling scale)."""
@@ -131,7 +135,7 @@ def _burnside_sq(Lx, Ly, n_up):
     return tot // (Lx * Ly)
 
 
-def test_square6x6_j1j2_k0_at_size():
+def test_square6x6_j1j2_k0_at_size(reference):
     from qed_spin_b200 import device as D
     Lx = Ly = 6
     nn, nnn = lat.square_j1j2_bonds(Lx, Ly)
@@ -163,7 +167,7 @@ def test_square6x6_j1j2_k0_at_size():
     assert np.array_equal(_bits(y_dev), _bits(y_ref))
 
 
-def test_ftlm_n24_blocks_against_reference():
+def test_ftlm_n24_blocks_against_reference(reference):
     from qed_spin_b200 import device as D
     N, seed = 24, 20240601
     betas = 1.0 / np.linspace(0.1, 4.0, 40)

@@ -6,6 +6,7 @@ enumeration's representatives depend on exactly these tables."""
 import numpy as np
 import pytest
 
+from conftest import need_reference
 from oracle import ref as R
 from qed_spin_b200 import lattice as lat
 
@@ -22,8 +23,7 @@ for _a, _b in ((4, 3), (4, 4), (5, 5), (6, 4), (6, 5), (6, 6), (8, 4), (8, 8)):
 @pytest.mark.parametrize("mode", [1, -1, -2, 0])
 @pytest.mark.parametrize("name,N,perms,flips", GROUPS, ids=[g[0] for g in GROUPS])
 def test_key_order_tables_equal_the_reference(name, N, perms, flips, mode):
-    if not R.available():
-        pytest.fail("the reference engine library is not built (oracle/Makefile, run by __graft_entry__.build())")
+    need_reference()
     from qed_spin_b200 import device as D
     spec = lat.SectorSpec(N, N // 2, np.asarray(perms, np.int32), np.ones(len(perms), np.complex128),
                           None if flips is None else np.asarray(flips, np.uint64))

@@ -4,13 +4,13 @@ size where the draw goes parallel and well past it (three million entries, a doz
 import numpy as np
 import pytest
 
+from conftest import need_reference
 from oracle import ref as R
 
 
 @pytest.mark.parametrize("seed,n", [(0x51ED0B70, 1000), (0x51ED900D, 3_000_000), (7, (1 << 20) + 1)])
 def test_staged_start_equals_the_reference_draw(seed, n):
-    if not R.available():
-        pytest.fail("the reference engine library is not built (oracle/Makefile, run by __graft_entry__.build())")
+    need_reference()
     from qed_spin_b200 import device as D
     mine = D.staged_start(seed, n)
     ref = R.staged_seed(seed, n)
