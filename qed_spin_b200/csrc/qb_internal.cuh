@@ -89,6 +89,10 @@ template <class F> int guarded(F&& f) {
 // calling thread's stream and the block is reused once it completes, so releasing never synchronises the device.
 void* dev_alloc(std::size_t bytes);
 void dev_free(void* p, std::size_t bytes);
+// Opts a kernel in to the most dynamic shared memory it can have beside its static arrays, once per kernel and device (the
+// same value whoever asks: a thread launching with fewer bytes does not lower another's; and asking the runtime at every
+// launch took 10 us of a small CSR's build).
+void allow_smem(const void* kernel);
 // A host-to-device copy that has completed on return; large pageable sources go through pinned slots (hostio.cu).
 void upload_host(void* dst, const void* src, std::size_t bytes, cudaStream_t st);
 std::size_t idle_cached_bytes();

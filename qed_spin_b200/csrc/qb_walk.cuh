@@ -143,19 +143,10 @@ inline std::size_t smem_for(const qb_program* P, const qb_sector* col, bool& in_
     return tables + (in_smem ? P->view.smem_bytes : 0);
 }
 
-// Lets a kernel be launched with `bytes` of dynamic shared memory. What needs no opt-in is 48 KB for its static arrays
-// and these together; the opt-in is for the most it can have, the same value whoever asks, so that a thread launching
-// with fewer bytes does not lower another's. (No kernel here has 40 KB of static arrays: below 8 KB nothing is asked.)
+// Lets a kernel be launched with `bytes` of dynamic shared memory: what needs no opt-in is 48 KB for its static arrays and
+// these together, and no kernel here has 40 KB of static arrays.
 template <class K> void set_smem(K kernel, std::size_t bytes) {
-    if (bytes <= 8 * 1024) return;
-    cudaFuncAttributes a;
-    cuda_check(cudaFuncGetAttributes(&a, kernel), "kernel attributes");
-    if (a.sharedSizeBytes + bytes <= 48 * 1024) return;
-    int dev = 0, most = 0;
-    cuda_check(cudaGetDevice(&dev), "device");
-    cuda_check(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev), "shared memory");
-    cuda_check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    most - static_cast<int>(a.sharedSizeBytes)), "smem attribute");
+    if (bytes > 8 * 1024) allow_smem(reinterpret_cast<const void*>(kernel));
 }
 
 }  // namespace qb

@@ -17,6 +17,7 @@
 #include <cstring>
 #include <mutex>
 #include <numeric>
+#include <set>
 
 #include "qb_canon.cuh"
 
@@ -37,6 +38,21 @@ std::size_t available_bytes() {
     if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) free_b = 0;
     free_b += idle_cached_bytes();   // released blocks the cache would hand out again
     return g_allowance ? std::min(free_b, g_allowance) : free_b;
+}
+
+void allow_smem(const void* kernel) {
+    static std::mutex mu;
+    static std::set<std::pair<const void*, int>> done;
+    int dev = 0, most = 0;
+    cuda_check(cudaGetDevice(&dev), "device");
+    std::lock_guard<std::mutex> lk(mu);
+    if (done.count({kernel, dev})) return;
+    cudaFuncAttributes a;
+    cuda_check(cudaFuncGetAttributes(&a, kernel), "kernel attributes");
+    cuda_check(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev), "shared memory");
+    cuda_check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    most - static_cast<int>(a.sharedSizeBytes)), "smem attribute");
+    done.insert({kernel, dev});
 }
 
 namespace {
@@ -860,9 +876,7 @@ int qb_sector_create(const qb_sector_desc* d, qb_sector** out) {
         DevBuf<u64> counts(n_chunks), offsets(n_chunks + 1);
         DSector v = s->view();
         const std::size_t smem = tables_smem_bytes(v);
-        if (smem > 48 * 1024)
-            cuda_check(cudaFuncSetAttribute(enum_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)),
-                       "smem attribute");
+        if (smem > 48 * 1024) allow_smem(reinterpret_cast<const void*>(enum_kernel));
         const unsigned threads = 256;
         const unsigned blocks =
             static_cast<unsigned>(std::min<u64>((n_chunks + threads - 1) / threads, static_cast<u64>(sm_count()) * 16));
@@ -954,9 +968,7 @@ int qb_index_and_projection(const qb_sector* s, const uint64_t* states, uint64_t
         DevBuf<long long> d_idx(n);
         DevBuf<double2> d_proj(n);
         const std::size_t smem = tables_smem_bytes(s->view());
-        if (smem > 48 * 1024)
-            cuda_check(cudaFuncSetAttribute(index_proj_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)),
-                       "smem attribute");
+        if (smem > 48 * 1024) allow_smem(reinterpret_cast<const void*>(index_proj_kernel));
         index_proj_kernel<<<static_cast<unsigned>((n + 127) / 128), 128, smem>>>(s->view(), d_states.p, n, d_idx.p,
                                                                                     d_proj.p);
         cuda_check(cudaGetLastError(), "index_and_projection");
