@@ -206,7 +206,8 @@ enum Cand : int { kLists = 0, kMasks = 1, kRowPairs = 2 };
 // brings it to row 0, row b + 1 behind it; the candidates are bits b Lx + a of one mask, read in order. The rows of a
 // 36-site state away from half filling tie often (an empty row ties with every other empty row under all its
 // rotations), and each tie costs an image and a comparison, for the slowest lane of the warp; pairs of rows hardly tie.
-// 6x6 at 11 spins up: 112 -> 70 ms per H.v (before, 11.5 lanes of a warp's 32 were active on average).
+// 6x6 at 11 spins up: 112 -> 58 ms per H.v (11.5 lanes of a warp's 32 were active on average before, 13.8 at 8 spins up
+// now).
 template <class ST, class Fn>
 __device__ __forceinline__ void for_each_row_candidate(const DSector& S, const u32* pair, ST t, Fn&& fn) {
     const int L = S.slc.L, m = S.slc.m;

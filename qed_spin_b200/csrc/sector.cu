@@ -571,8 +571,9 @@ int classify_group(const int32_t* perms, int G, int N, int& Lx, std::vector<u64>
 }
 
 // The row-pair table (for_each_row_candidate) when the group is every translation of a torus, numbered a + Lx b and
-// without flips, and the key order's blocks are its rows, of at most 6 sites (16 KB), with more than 32 sites (the
-// kernels of 32-bit states, chains above all, stay without the second kind of candidate): entry (first | second << L) holds
+// without flips, and the key order's blocks are its rows, of at most 6 sites (16 KB), with more than 32 sites (32-bit states
+// collect masks or read lists). Of the tori of 33 to 64 sites that is 6x6 alone: the key order takes the largest blocks of at
+// most 16 sites, which are single rows of at most 6 sites on no other: entry (first | second << L) holds
 // the least (rot_a first << L | rot_a second) over the rotations a, << 8, and the rotations that reach it.
 void build_pair_table(qb_sector& s, const qb_sector_desc& d, QueuedUploads& up) {
     const int L = s.slc_L, m = s.slc_m;
