@@ -1074,6 +1074,8 @@ void ftlm_blocks(const qb_sector* const* secs, const qb_program* const* progs, i
         }
         dG.alloc(G.size());
         cuda_check(cudaMemcpy(dG.p, G.data(), G.size() * 16, cudaMemcpyHostToDevice), "samples upload");
+        // the copy from pageable memory may still be under way when the call returns, and the blocks' streams wait for no other
+        cuda_check(cudaStreamSynchronize(cudaStreamPerThread), "samples upload");
     }
     st_draw = secs_since(t_phase);
     // blocks, largest first, dealt round robin to a few streams so small blocks overlap
