@@ -1215,9 +1215,7 @@ void ftlm_blocks(const qb_sector* const* secs, const qb_program* const* progs, i
     cuda_check(cudaMemsetAsync(err.p, 0, 4, st0), "zero");
     const int cthreads = in_smem ? 32 : 128;
     const std::size_t csmem = in_smem ? row_bytes * 32 : 0;
-    if (csmem > 48 * 1024)
-        cuda_check(cudaFuncSetAttribute(k_sample_moments, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        static_cast<int>(csmem)), "smem attribute");
+    if (csmem > 48 * 1024) allow_smem(reinterpret_cast<const void*>(k_sample_moments));
     k_sample_moments<<<(n_items + cthreads - 1) / cthreads, cthreads, csmem, st0>>>(
         d_cb.p, n_items, k, d_alpha.p, d_beta.p, d_betas.p, n_beta, cap_max, in_smem, scratch.p, ord.p, mom.p, err.p);
     const std::size_t n_comb = static_cast<std::size_t>(n_blocks) * std::max(1, n_beta);
