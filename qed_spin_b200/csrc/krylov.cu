@@ -1147,6 +1147,16 @@ void ftlm_blocks(const qb_sector* const* secs, const qb_program* const* progs, i
                 if (c) qb_csr_destroy(c);
         }
     } csrs{std::vector<qb_csr*>(n_blocks, nullptr)};
+    // left by an exception: the queued steps end before the buffers and matrices above go back to the block cache, which knows
+    // of this thread's stream alone
+    struct Drain {
+        const std::vector<cudaStream_t>& s;
+        cudaStream_t pack;
+        ~Drain() {
+            for (auto st : s) cudaStreamSynchronize(st);
+            cudaStreamSynchronize(pack);
+        }
+    } drain{streams, pst};
     t_phase = clock::now();
     if (use_csr) {
         // the builds synchronise with the host a few times each: a few host threads, each on its own stream, keep
