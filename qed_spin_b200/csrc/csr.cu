@@ -1077,6 +1077,9 @@ void build_slices(qb_csr* A, uint64_t max_bytes) {
     k_slice<<<static_cast<unsigned>((A->rows + 255) / 256), 256>>>(A->rows, A->row_ptr.p, A->col_idx.p, A->ids.p, cb,
                                                                    A->slices.p);
     cuda_check(cudaGetLastError(), "CSR slices");
+    // asks for the kernels' occupancies now: the first apply may be under capture
+    sliced_form<true, true>(A);
+    sliced_form<true, false>(A);
 }
 
 // ... and at most this much scratch, an eighth of the free memory at most, and what a server's worker was admitted with.

@@ -2,9 +2,13 @@
 sliced copy): FP64 storage bit for bit, FP32 storage within the rounding of its output (1.2e-7). Row counts that are no
 multiple of a slice or a block, rows of 1 to 75 entries, complex values, a matrix between two sectors, and row counts on
 both sides of each form's last wave; and the same copy whichever way the matrix was built."""
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
+from conftest import ROOT
 from qed_spin_b200 import lattice as lat
 from qed_spin_b200 import operators as ops
 
@@ -84,3 +88,27 @@ def test_slices_of_a_matrix_built_the_general_way():
     A.matvec(x, y, dtype="c64")
     B.matvec(x, z, dtype="c64")
     assert torch.equal(torch.view_as_real(y).view(torch.int32), torch.view_as_real(z).view(torch.int32))
+
+
+@pytest.mark.parametrize("dtype", ["c64", "c128"])
+def test_first_apply_of_a_process_under_capture(dtype):
+    """A process whose first sliced apply is captured in a graph: the replay equals the apply."""
+    code = f"""
+import sys
+import torch
+from qed_spin_b200 import device as D, lattice as lat, operators as ops
+S = D.Sector(lat.chain_sector(24, 11, 5))
+A = D.Csr(S, S, D.Program(ops.row_program(ops.from_products(24, ops.heisenberg_products(lat.chain_bonds(24))))))
+x = torch.randn(S.dim, dtype=torch.{'complex64' if dtype == 'c64' else 'complex128'}, device="cuda")
+y, z = torch.zeros_like(x), torch.empty_like(x)
+torch.cuda.synchronize()
+g = torch.cuda.CUDAGraph()
+with torch.cuda.graph(g):
+    A.matvec(x, y, dtype="{dtype}", stream=torch.cuda.current_stream())
+g.replay()
+A.matvec(x, z, dtype="{dtype}", stream=torch.cuda.current_stream())
+torch.cuda.synchronize()
+sys.exit(0 if torch.equal(y, z) and float(y.abs().max()) > 0 else 1)
+"""
+    r = subprocess.run([sys.executable, "-c", code], cwd=ROOT, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
